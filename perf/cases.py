@@ -6,6 +6,7 @@
     run(state)          one call, as a program makes it, and its outputs
     work(case)          bytes and operations one call cannot do without
     tolerance(case)     how far another correct implementation of the same precision may be
+    exact(case, seed)   the outputs of that call in 64 bits
 
 Kinds of case ("op"):
 
@@ -185,3 +186,45 @@ def tolerance(case):
     if case["op"] == "rope":
         return {"rel": 2e-3, "max": 3e-2}
     return {"rel": 6e-3, "max": 2e-2}
+
+
+def _dequantised(t, s, row_block):
+    """t * its block scales in 64 bits: one scale per `row_block` rows and 128 columns."""
+    rows = torch.arange(t.shape[-2], device=t.device) // row_block
+    return t.double() * s.double().index_select(-2, rows).repeat_interleave(128, dim=-1)
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, evaluated in 64 bits."""
+    s = prepare(case, seed)
+    op = case["op"]
+    if op == "kv_down":
+        return _dequantised(s["x"], s["xs"], 1) @ _dequantised(s["w"], s["ws"], 128).t()
+    if op in ("gemm", "host"):
+        a, b, a_s, b_s, _ = (t.to(DEV) for t in (s["data"] if op == "gemm" else s["args"]))
+        c = _dequantised(a, a_s, 1) @ _dequantised(b, b_s, 128).t()
+        return c.cpu() if op == "host" else c
+    if op == "grouped":
+        a, b, a_s, b_s, c = s["args"]
+        out = torch.zeros(c.shape, dtype=torch.float64, device=DEV)
+        for g, r in enumerate(s["rows"].tolist()):  # rows past a group's count keep what c held: zeros
+            out[g, :r] = _dequantised(a[g, :r], a_s[g, :r], 1) @ _dequantised(b[g], b_s[g], 128).t()
+        return out
+    if op == "softmax":
+        return torch.softmax(s["qk"].double() / math.sqrt(DNOPE + DROPE), dim=-1)
+    # The angles' bf16 steps belong to the operator (a position of 6144 has a bf16 step of 32): they are taken as
+    # they are, the trigonometry and the rotation in 64 bits.
+    half = DROPE // 2
+    exponent = ((torch.arange(half, device=DEV).bfloat16() * -2.0).float() / DROPE).bfloat16()
+    base = torch.pow(torch.tensor(10000.0, device=DEV).bfloat16().double(), exponent.double()).bfloat16()
+
+    def rotated(x, pos, n):
+        idx = (torch.tensor(float(pos)).bfloat16().to(DEV).float() + torch.arange(n, device=DEV).bfloat16().float()).bfloat16()
+        theta = (idx.float()[:, None] * base.float()[None, :]).bfloat16().double()
+        x = x.double()
+        lo, hi = x[..., :half], x[..., half:]
+        return torch.cat((lo * theta.cos() - hi * theta.sin(), hi * theta.cos() + lo * theta.sin()), dim=-1)
+
+    q = s["q"].double()
+    q[..., DNOPE:] = rotated(s["q"][..., DNOPE:], s["sl"] - 1, 1)
+    return q, rotated(s["cache"][..., DKV:], 0, s["sl"])
