@@ -64,54 +64,62 @@ __global__ void __launch_bounds__(256) rope_kernel(const __nv_bfloat16* __restri
   }
 }
 
-constexpr int kRopeTable = 256;  // pair indices whose 10000^(-2j/d2) a CTA keeps in shared memory
+constexpr int kRopeThreads = 256;
+constexpr int kRopeTable = 256;     // pair indices whose 10000^(-2j/d2) a CTA keeps in shared memory
+constexpr int kRopeWidePairs = 16384;  // from here on a CTA takes kRopeMaxUnits units
+constexpr int kRopeMaxUnits = 256;  // units (position, eight adjacent pair indices) of one CTA
 
 // The same with eight adjacent pair indices per thread: 16-byte loads and stores. Used when d2/2 is a multiple of 8
 // and every row start is 16-byte aligned (checked by the launcher).
-__global__ void __launch_bounds__(256) rope_kernel_vec8(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* y, int pos,
-                                                        int d0, int d1, int d2, long long xs1, long long xs2,
-                                                        long long ys1, long long ys2, int rows_per_block) {
+//
+// Bound by HBM (2 bytes in, 2 out per element). A CTA owns `units` (a power of two) units of eight pair indices and a
+// range of d0 rows, walked 256 / units rows at a time. The angles are a function of the unit alone: the CTA evaluates
+// each once into shared memory, all threads sharing that work, and every row reads them from there. So a small d1 (the
+// query of a decode step: one position, four units) still runs with every thread busy on a row of its own, and a large
+// d1 can be cut into many short CTAs without paying for the trigonometry again in each thread.
+__global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* y,
+                                                                 int pos, int d0, int d1, int d2, long long xs1,
+                                                                 long long xs2, long long ys1, long long ys2, int units,
+                                                                 int rows_per_block) {
   const int half = d2 >> 1;
-  const int groups = half >> 3;  // groups of eight pair indices per position row
-  // 10000^(-2j/d2) depends on j alone: the CTA computes the table once (powf is about half of a thread's angle
-  // arithmetic) when it fits; every thread then needs only a cosf and a sinf per pair index.
+  const int groups = half >> 3;  // units per position
   __shared__ __nv_bfloat16 base_tab[kRopeTable];
+  __shared__ __align__(16) __nv_bfloat16 cos_tab[kRopeMaxUnits * 8];
+  __shared__ __align__(16) __nv_bfloat16 sin_tab[kRopeMaxUnits * 8];
+  const int tid = static_cast<int>(threadIdx.x);
+  const long long total = static_cast<long long>(d1) * groups;
+  const long long first = static_cast<long long>(blockIdx.x) * units;
   const bool use_tab = half <= kRopeTable;
   if (use_tab) {
-    for (int j = threadIdx.x; j < half; j += blockDim.x) base_tab[j] = rope_base(j, d2);
+    for (int j = tid; j < half; j += kRopeThreads) base_tab[j] = rope_base(j, d2);
     __syncthreads();
   }
-  const long long g = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (g >= static_cast<long long>(d1) * groups) return;
+  for (int a = tid; a < units * 8; a += kRopeThreads) {
+    const long long g = first + (a >> 3);
+    if (g >= total) break;
+    const int i1 = static_cast<int>(g / groups);
+    const int j = static_cast<int>(g - static_cast<long long>(i1) * groups) * 8 + (a & 7);
+    rope_rotation(use_tab ? base_tab[j] : rope_base(j, d2), pos, i1, &cos_tab[a], &sin_tab[a]);
+  }
+  __syncthreads();
+  const int unit = tid & (units - 1);
+  const long long g = first + unit;
+  if (g >= total) return;
   const int i1 = static_cast<int>(g / groups);
   const int j0 = static_cast<int>(g - static_cast<long long>(i1) * groups) * 8;
-  __nv_bfloat16 c[8], s[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    __nv_bfloat16 ce, se;
-    rope_rotation(use_tab ? base_tab[j0 + e] : rope_base(j0 + e, d2), pos, i1, &ce, &se);
-    c[e] = ce;
-    s[e] = se;
-  }
-  const int r0 = blockIdx.y * rows_per_block;
+  const int step = kRopeThreads / units;
+  const int r0 = static_cast<int>(blockIdx.y) * rows_per_block;
   const int r1 = min(d0, r0 + rows_per_block);
   const __nv_bfloat16* xp = x + static_cast<long long>(i1) * xs2 + j0;
   __nv_bfloat16* yp = y + static_cast<long long>(i1) * ys2 + j0;
-  // Four rows at a time: their eight 16-byte loads are issued before the first result is stored, so a thread keeps
-  // 128 bytes in flight instead of 32 (in place is still fine: a row's loads precede its own stores, and rows do
-  // not overlap).
-  constexpr int kRowsInFlight = 4;
   // The rotation in packed bf16 arithmetic (two elements per instruction). The hardware's bf16 multiply, add and
   // subtract round the exact result once; rounding the fp32 result of the same operation to bf16, which is what
   // the reference's arithmetic amounts to, gives the same value (a bf16 product is exact in fp32, and fp32 carries
   // more than twice bf16's precision plus two bits, so the double rounding of a sum is harmless). The _rn forms
   // are never contracted into a fused multiply-add, which would skip the products' rounding.
   __nv_bfloat162 c2[4], s2[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    c2[e] = __halves2bfloat162(c[2 * e], c[2 * e + 1]);
-    s2[e] = __halves2bfloat162(s[2 * e], s[2 * e + 1]);
-  }
+  *reinterpret_cast<uint4*>(c2) = *reinterpret_cast<const uint4*>(cos_tab + unit * 8);
+  *reinterpret_cast<uint4*>(s2) = *reinterpret_cast<const uint4*>(sin_tab + unit * 8);
   auto rotate_store = [&](const uint4& a, const uint4& b, int i0) {
     const __nv_bfloat162* x1 = reinterpret_cast<const __nv_bfloat162*>(&a);
     const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&b);
@@ -126,18 +134,22 @@ __global__ void __launch_bounds__(256) rope_kernel_vec8(const __nv_bfloat16* __r
     *reinterpret_cast<uint4*>(yp + i0 * ys1) = o1;
     *reinterpret_cast<uint4*>(yp + i0 * ys1 + half) = o2;
   };
-  int i0 = r0;
-  for (; i0 + kRowsInFlight <= r1; i0 += kRowsInFlight) {
+  // Four rows at a time: their eight 16-byte loads are issued before the first result is stored, so a thread keeps
+  // 128 bytes in flight instead of 32 (in place is still fine: a row's loads precede its own stores, and rows do
+  // not overlap).
+  constexpr int kRowsInFlight = 4;
+  int i0 = r0 + tid / units;
+  for (; i0 + (kRowsInFlight - 1) * step < r1; i0 += kRowsInFlight * step) {
     uint4 a[kRowsInFlight], b[kRowsInFlight];
 #pragma unroll
     for (int u = 0; u < kRowsInFlight; ++u) {
-      a[u] = *reinterpret_cast<const uint4*>(xp + (i0 + u) * xs1);
-      b[u] = *reinterpret_cast<const uint4*>(xp + (i0 + u) * xs1 + half);
+      a[u] = *reinterpret_cast<const uint4*>(xp + (i0 + u * step) * xs1);
+      b[u] = *reinterpret_cast<const uint4*>(xp + (i0 + u * step) * xs1 + half);
     }
 #pragma unroll
-    for (int u = 0; u < kRowsInFlight; ++u) rotate_store(a[u], b[u], i0 + u);
+    for (int u = 0; u < kRowsInFlight; ++u) rotate_store(a[u], b[u], i0 + u * step);
   }
-  for (; i0 < r1; ++i0) {
+  for (; i0 < r1; i0 += step) {
     const uint4 a = *reinterpret_cast<const uint4*>(xp + i0 * xs1);
     const uint4 b = *reinterpret_cast<const uint4*>(xp + i0 * xs1 + half);
     rotate_store(a, b, i0);
@@ -295,23 +307,36 @@ int b200_mla_rope(const void* x, void* y, int pos, int d0, int d1, int d2, long 
   const bool vec8 = (half % 8) == 0 && (xs1 % 8) == 0 && (xs2 % 8) == 0 && (ys1 % 8) == 0 && (ys2 % 8) == 0 &&
                     (reinterpret_cast<uintptr_t>(x) % 16) == 0 && (reinterpret_cast<uintptr_t>(y) % 16) == 0;
   const long long pairs = static_cast<long long>(d1) * (vec8 ? half / 8 : half);
-  const int threads = 256;
-  const long long blocks_x = (pairs + threads - 1) / threads;
+  // Units per CTA of the 16-byte kernel. Many units (the keys of a whole cache): as wide a CTA as there is, so that
+  // the CTAs running together sweep few rows from end to end, which HBM likes best (6145 positions x 128 rows: 256
+  // units 38 us, 32 to 128 units 41 to 45). Fewer: 32, so that there are CTAs for every SM (2049 positions x 32 rows:
+  // 5.2 against 6.1 us). Never more threads for the units than rows leave idle, never fewer units than one per row
+  // slot, and more where the grid would otherwise pass its limit.
+  long long units = kRopeThreads;
+  if (vec8 && pairs < kRopeWidePairs) {
+    units = 1;
+    while (units < pairs && units < 32) units *= 2;
+    while (units < kRopeMaxUnits && kRopeThreads / units > d0) units *= 2;
+  }
+  const int ctas_per_sm = (vec8 && units < kRopeMaxUnits) ? 4 : 2;
+  const long long blocks_x = (pairs + units - 1) / units;
   if (blocks_x > 0x7fffffffll) return B200_FP8_MM_ERR_SHAPE;
-  // enough CTAs for every SM a few times over, without cutting d0 finer than 4 rows per CTA
-  long long want_y = (148 * 2 + blocks_x - 1) / blocks_x;
-  if (want_y > (d0 + 3) / 4) want_y = (d0 + 3) / 4;
+  // Rows per CTA: CTAs for every SM a few times over (each evaluates its units' angles once).
+  const int row_step = vec8 ? static_cast<int>(kRopeThreads / units) : 1;
+  const int min_rows = row_step > 4 ? row_step : 4;
+  long long want_y = (148 * ctas_per_sm + blocks_x - 1) / blocks_x;
+  if (want_y > (d0 + min_rows - 1) / min_rows) want_y = (d0 + min_rows - 1) / min_rows;
   if (want_y < 1) want_y = 1;
   if (want_y > 65535) want_y = 65535;
-  const int rows_per_block = static_cast<int>((d0 + want_y - 1) / want_y);
-  const int blocks_y = (d0 + rows_per_block - 1) / rows_per_block;
+  const int rows_per_block = static_cast<int>(((d0 + want_y - 1) / want_y + row_step - 1) / row_step * row_step);
+  const int blocks_y = static_cast<int>((static_cast<long long>(d0) + rows_per_block - 1) / rows_per_block);
   const dim3 grid(static_cast<unsigned>(blocks_x), static_cast<unsigned>(blocks_y));
   if (vec8) {
-    rope_kernel_vec8<<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(
+    rope_kernel_vec8<<<grid, kRopeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), pos, d0, d1, d2, xs1, xs2, ys1, ys2,
-        rows_per_block);
+        static_cast<int>(units), rows_per_block);
   } else {
-    rope_kernel<<<grid, threads, 0, static_cast<cudaStream_t>(stream)>>>(
+    rope_kernel<<<grid, kRopeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), pos, d0, d1, d2, xs1, xs2, ys1, ys2,
         rows_per_block);
   }
