@@ -64,6 +64,7 @@ constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // default limit of 
 constexpr int kCounterBytes = 4096;
 constexpr int kMaxCounters = kCounterBytes / 4;
 constexpr int kMaxStages = 8;
+constexpr int kMaxCluster = 8;  // CTAs per thread-block cluster that every device accepts without opting in to more
 constexpr int kStoreBoxCols = 32;                                // bf16 columns per TMA store box (64 bytes)
 constexpr int kStoreBufBytes = kBlockM * kStoreBoxCols * 2;      // one staging buffer: 128 rows x 64 B
 constexpr int kScaleGroup = 4;  // K blocks per scale-ring slot (4 or 8; 8 measured no faster, 10 % slower at BN=128)
@@ -138,6 +139,16 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// 16 bytes of a cluster CTA's shared memory (shared::cluster address).
+__device__ __forceinline__ float4 ld_cluster(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -619,7 +630,9 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
 // GENERIC = false is the plain case (K-major a and b, one problem): operand layout and work list are
 // compile-time facts and none of the MN-major / grouped code is in the instruction stream of the
 // single-thread roles, whose per-K-block instruction count is on the critical path of narrow tiles.
-template <int BN, bool PAIR, bool GENERIC>
+// CLUSTER: the K ranges of a tile are the CTAs of one thread-block cluster (cluster rank = range, one work item per
+// CTA) and the reduction goes through their shared memory; see the end of the kernel.
+template <int BN, bool PAIR, bool GENERIC, bool CLUSTER = false>
 __global__ void __launch_bounds__((TileCfg<BN, PAIR>::kThreads), 1)
 fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                           const __grid_constant__ CUtensorMap tmap_c, const KernelParams p) {
@@ -1071,6 +1084,18 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           acc[j] = unpack2(acc2[j]);
         }
       }
+      if constexpr (CLUSTER) {
+        // This K range's fp32 tile goes to the operand ring, which nothing uses any more: every K block this CTA
+        // loaded has been multiplied (its done barrier was waited for above). Rows BN + 4 floats apart, so that a
+        // quarter warp's 16-byte stores cover all banks.
+        if (ok && row < p.M) {
+          float4* mine = reinterpret_cast<float4*>(ring + static_cast<size_t>(row_in_tile) * (BN + 4) * 4) + (col_base >> 2);
+#pragma unroll
+          for (int j = 0; j < Cfg::kColsPerThread / 4; ++j)
+            mine[j] = make_float4(acc[2 * j].x, acc[2 * j].y, acc[2 * j + 1].x, acc[2 * j + 1].y);
+        }
+        continue;
+      }
       const int col0 = it.n0 + col_base;  // first column of this thread inside (the shard of) c
       bool do_store = true;  // the same in every promotion thread of the CTA
       if (it.nsplit > 1) {
@@ -1277,6 +1302,53 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     }
   }
 
+  if constexpr (CLUSTER) {
+    // Split-K reduction inside the cluster. Every CTA's partial tile lies in its own shared memory; the existing rows
+    // are dealt out to all promotion threads of the cluster in pieces of four columns, each thread reads its piece
+    // from every CTA (all loads in flight together), adds them in order 0..ranges-1 and stores
+    // bf16. No fp32 plane, counter or fence goes through global memory: on 128 x 576 x 7168 the reduction through the
+    // planes took about 5 of 12 us, most of it one CTA reading all sixteen planes of a tile by itself.
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 4 && *abort_flag == 0) {
+      const int ranges = p.split_k;
+      const WorkItem it = decode_work<GENERIC>(p, static_cast<int>(blockIdx.x), Cfg::kTileM, BN);
+      constexpr int kPieces = BN / 4;  // per row
+      const int rows = min(kBlockM, p.M - it.m0);
+      const uint32_t base = smem_u32(ring);
+      for (int u = it.split * Cfg::kEpiThreads + static_cast<int>(threadIdx.x) - 128; u < rows * kPieces;
+           u += ranges * Cfg::kEpiThreads) {
+        const int r = u / kPieces, col = (u % kPieces) * 4;
+        const uint32_t at = base + static_cast<uint32_t>(r * (BN + 4) + col) * 4u;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 t[kMaxCluster];
+#pragma unroll
+        for (int s = 0; s < kMaxCluster; ++s)
+          if (s < ranges) t[s] = ld_cluster(map_to_cta(at, static_cast<uint32_t>(s)));
+#pragma unroll
+        for (int s = 0; s < kMaxCluster; ++s)
+          if (s < ranges) {
+            sum.x += t[s].x;
+            sum.y += t[s].y;
+            sum.z += t[s].z;
+            sum.w += t[s].w;
+          }
+        __nv_bfloat16* dst = p.c + static_cast<long long>(it.m0 + r) * p.ldc + it.n0 + col;
+        const int cols = p.N - (it.n0 + col);
+        const uint32_t lo = pack_bf16x2(sum.x, sum.y), hi = pack_bf16x2(sum.z, sum.w);
+        if (cols >= 4 && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
+          *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
+        } else {
+          unsigned short* d16 = reinterpret_cast<unsigned short*>(dst);
+          if (cols > 0) d16[0] = static_cast<unsigned short>(lo);
+          if (cols > 1) d16[1] = static_cast<unsigned short>(lo >> 16);
+          if (cols > 2) d16[2] = static_cast<unsigned short>(hi);
+          if (cols > 3) d16[3] = static_cast<unsigned short>(hi >> 16);
+        }
+      }
+    }
+    __syncwarp();
+  }
   if (warp >= 4) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");  // none in flight past here
     // the staging buffers must outlive the bulk stores that read them
@@ -1286,7 +1358,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   // CTA may exit while its peer can still signal its barriers or use its shared memory.
   tcgen05_fence_before();
   __syncthreads();
-  if constexpr (PAIR) cluster_sync_all();
+  // (and no CTA of a split-K cluster while a peer reads its partial tile)
+  if constexpr (PAIR || CLUSTER) cluster_sync_all();
   if (warp == 2) {
     tcgen05_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_base_slot);
@@ -1571,6 +1644,34 @@ double pair_penalty(int bn, int split) {
   return 1.04;
 }
 
+// Clusters of one-CTA-per-SM kernels that are on the device together, by cluster size, as
+// cudaOccupancyMaxActiveClusters answers on B200 (148 SMs; a cluster stays inside one GPC). More clusters than that are
+// correct and take a second wave.
+int cluster_capacity(int ctas, int sm_count) {
+  static const int at148[kMaxCluster + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+  return static_cast<int>(static_cast<long long>(at148[ctas]) * sm_count / 148);
+}
+
+// Whether a split plan's ranges run as thread-block clusters (see the kernel's CLUSTER parameter): every tile is
+// split, the clusters are on the device together, and the operand ring can hold a tile's fp32 partials. A second wave
+// of clusters costs more than the planes: 256 x 1536 x 7168 as 48 clusters of three 20.4 us, through the planes 13.6.
+bool runs_as_cluster(const b200_fp8_mm_plan& pl, int sm_count) {
+  if (pl.cta_pair || pl.full_tiles != 0 || pl.split_k < 2 || pl.split_k > kMaxCluster) return false;
+  if (pl.block_n != 64 && pl.block_n != 128) return false;
+  if (pl.tiles > cluster_capacity(pl.split_k, sm_count)) return false;
+  return pl.stages * (kBlockM + pl.block_n) * kBlockK >= kBlockM * (pl.block_n + 4) * 4;
+}
+
+// Cost of a split plan that runs as clusters, in the selector's clocks, fitted to timings of every such plan over 28
+// problems of 16 to 512 rows (K 512 to 7168). Beside the K blocks of one range there is a constant for the cluster
+// launch and its two barriers, and the reduction, which grows with the rows a tile really has.
+double cluster_cost(int M, int kblocks, int bn, int split) {
+  const double rows = (M < kBlockM ? M : kBlockM) / static_cast<double>(kBlockM);
+  const int kb = (kblocks + split - 1) / split;
+  if (bn == 64) return kb * 400.0 + 1850.0 + 2600.0 + 360.0 * split * (0.5 + 0.5 * rows);
+  return kb * 480.0 + 2800.0 + 2500.0 + 1200.0 * rows + 450.0 * split;
+}
+
 struct Candidate {
   int bn, pair, split, full_tiles;
   double cost;
@@ -1617,23 +1718,9 @@ Candidate evaluate(int M, int N, int kblocks, int sm_count, int bn, int pair, in
   return best;
 }
 
-double choose_plan(int M, int N, int K, int sm_count, const b200_fp8_mm_plan* forced, b200_fp8_mm_plan* out) {
-  const int kblocks = K / kBlockK;
-  const int f_bn = (forced && forced->block_n) ? forced->block_n : 0;
-  const int f_pair = (forced && forced->cta_pair) ? (forced->cta_pair > 0 ? 1 : 0) : -1;  // -1: choose
-  const int f_split = (forced && forced->split_k) ? forced->split_k : 0;
-  Candidate best{0, 0, 1, 0, 1e300};
-  const int cands[4] = {256, 192, 128, 64};
-  for (int pair = 1; pair >= 0; --pair) {
-    if (f_pair >= 0 && pair != f_pair) continue;
-    if (f_pair < 0 && pair == 1 && M <= kBlockM) continue;  // a pair needs two row blocks to be useful
-    for (int i = 0; i < 4; ++i) {
-      if (f_bn && cands[i] != f_bn) continue;
-      const Candidate c = evaluate(M, N, kblocks, sm_count, cands[i], pair, f_split);
-      if (c.cost < best.cost - 1e-9) best = c;
-    }
-  }
-  if (best.bn == 0) best = Candidate{f_bn, f_pair > 0 ? 1 : 0, 1, 0, 0.0};  // invalid forced width
+// The launch plan of a candidate.
+void fill_plan(int M, int N, int kblocks, int sm_count, const b200_fp8_mm_plan* forced, const Candidate& best,
+               b200_fp8_mm_plan* out) {
   const int pair = best.pair;
   const int bn = best.bn;
   const int tiles = ceil_div(M, pair ? 2 * kBlockM : kBlockM) * ceil_div(N, bn > 0 ? bn : 1);
@@ -1657,6 +1744,47 @@ double choose_plan(int M, int N, int K, int sm_count, const b200_fp8_mm_plan* fo
   out->grid = pair ? 2 * used : used;
   out->store_bufs = store_bufs;
   out->smem_bytes = valid_block_n(bn) ? smem_bytes_for(bn, stages, pair, store_bufs) : 0;
+}
+
+double choose_plan(int M, int N, int K, int sm_count, const b200_fp8_mm_plan* forced, b200_fp8_mm_plan* out,
+                   size_t* workspace_need = nullptr) {
+  const int kblocks = K / kBlockK;
+  const int f_bn = (forced && forced->block_n) ? forced->block_n : 0;
+  const int f_pair = (forced && forced->cta_pair) ? (forced->cta_pair > 0 ? 1 : 0) : -1;  // -1: choose
+  const int f_split = (forced && forced->split_k) ? forced->split_k : 0;
+  Candidate best{0, 0, 1, 0, 1e300};
+  const int cands[4] = {256, 192, 128, 64};
+  for (int pair = 1; pair >= 0; --pair) {
+    if (f_pair >= 0 && pair != f_pair) continue;
+    if (f_pair < 0 && pair == 1 && M <= kBlockM) continue;  // a pair needs two row blocks to be useful
+    for (int i = 0; i < 4; ++i) {
+      if (f_bn && cands[i] != f_bn) continue;
+      const Candidate c = evaluate(M, N, kblocks, sm_count, cands[i], pair, f_split);
+      if (c.cost < best.cost - 1e-9) best = c;
+    }
+  }
+  if (best.bn == 0) best = Candidate{f_bn, f_pair > 0 ? 1 : 0, 1, 0, 0.0};  // invalid forced width
+  fill_plan(M, N, kblocks, sm_count, forced, best, out);
+  // What the caller's workspace must hold is decided by this plan. Running the ranges as clusters needs none, so a
+  // cluster plan that is cheaper replaces it without asking for more.
+  if (workspace_need != nullptr) *workspace_need = plan_workspace_bytes(*out);
+  if (f_split == 0 && f_pair <= 0 && valid_block_n(best.bn)) {
+    for (int bn = 64; bn <= 128; bn += 64) {
+      if (f_bn && bn != f_bn) continue;
+      const int tiles = ceil_div(M, kBlockM) * ceil_div(N, bn);
+      for (int split = 2; split <= kMaxCluster && split * 2 <= kblocks; ++split) {
+        if (tiles > cluster_capacity(split, sm_count)) break;
+        const double cost = cluster_cost(M, kblocks, bn, split);
+        if (cost >= best.cost) continue;
+        const Candidate c{bn, 0, split, 0, cost};
+        b200_fp8_mm_plan pl;
+        fill_plan(M, N, kblocks, sm_count, forced, c, &pl);
+        if (!runs_as_cluster(pl, sm_count)) continue;
+        best = c;
+        *out = pl;
+      }
+    }
+  }
   return best.cost;
 }
 
@@ -1688,7 +1816,12 @@ bool plan_is_supported(const b200_fp8_mm_plan& pl, int kblocks) {
 typedef void (*KernelFn)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const KernelParams);
 
 // generic: MN-major operands or a grouped launch (CTA pairs at the 192- and 256-wide tiles only).
-KernelFn kernel_for(int block_n, int pair, bool generic) {
+KernelFn kernel_for(int block_n, int pair, bool generic, bool cluster = false) {
+  if (cluster) {
+    if (block_n == 64) return generic ? fp8_mm_blockscaled_kernel<64, false, true, true> : fp8_mm_blockscaled_kernel<64, false, false, true>;
+    if (block_n == 128) return generic ? fp8_mm_blockscaled_kernel<128, false, true, true> : fp8_mm_blockscaled_kernel<128, false, false, true>;
+    return nullptr;
+  }
   if (generic) {
     if (pair) {
       // grouped launches on the two widths where pairs pay
@@ -1737,7 +1870,7 @@ int sm_count_for_sizing() {
   return n > 0 ? n : 148;
 }
 
-int launch(KernelFn fn, const b200_fp8_mm_plan& pl, const CUtensorMap& map_a, const CUtensorMap& map_b,
+int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUtensorMap& map_a, const CUtensorMap& map_b,
            const CUtensorMap& map_c, const KernelParams& kp, void* stream);
 
 // Storage of one fp8 operand from its two element strides: K-major (k stride 1) or MN-major (row stride 1).
@@ -1792,7 +1925,8 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   };
   const b200_fp8_mm_plan* forced = forced_in;
   b200_fp8_mm_plan pl;
-  choose_plan(M, N, K, sm_count, forced, &pl);
+  size_t need = 0;
+  choose_plan(M, N, K, sm_count, forced, &pl, &need);
   b200_fp8_mm_plan forced_copy;
   if (!pair_plan_runs(pl)) {
     if (forced_in != nullptr && forced_in->cta_pair > 0) return B200_FP8_MM_ERR_PLAN;
@@ -1803,16 +1937,17 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
     }
     forced_copy.cta_pair = -1;
     forced = &forced_copy;
-    choose_plan(M, N, K, sm_count, forced, &pl);
+    choose_plan(M, N, K, sm_count, forced, &pl, &need);
   }
   const int kblocks = K / kBlockK;
   if (!plan_is_supported(pl, kblocks)) return B200_FP8_MM_ERR_PLAN;
-  const size_t need = plan_workspace_bytes(pl);
   if (need > 0 && (workspace == nullptr || workspace_bytes < need ||
                    (reinterpret_cast<uintptr_t>(workspace) % 256) != 0))
     return B200_FP8_MM_ERR_WORKSPACE;
 
-  KernelFn fn = kernel_for(pl.block_n, pl.cta_pair, generic);
+  const bool cluster = runs_as_cluster(pl, sm_count);
+  if (cluster) pl.grid = pl.tiles * pl.split_k;
+  KernelFn fn = kernel_for(pl.block_n, pl.cta_pair, generic, cluster);
   if (fn == nullptr) return B200_FP8_MM_ERR_PLAN;
 
   CUtensorMap map_a, map_b, map_c;
@@ -1892,19 +2027,20 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
       return B200_FP8_MM_ERR_LAUNCH;
     }
   }
-  return launch(fn, pl, map_a, map_b, map_c, kp, stream);
+  return launch(fn, pl, cluster ? pl.split_k : (pl.cta_pair ? 2 : 1), map_a, map_b, map_c, kp, stream);
 }
 
-int launch(KernelFn fn, const b200_fp8_mm_plan& pl, const CUtensorMap& map_a, const CUtensorMap& map_b,
+int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUtensorMap& map_a, const CUtensorMap& map_b,
            const CUtensorMap& map_c, const KernelParams& kp, void* stream) {
   // Opt every kernel in to the full 227 KiB of dynamic shared memory once per device.
   cudaError_t err = cudaSuccess;
   {
-    static unsigned char opted_in[64][16] = {};
+    static unsigned char opted_in[64][32] = {};
     int dev = 0;
     (void)cudaGetDevice(&dev);
     const bool generic = kp.groups > 0 || kp.a_mn || kp.b_mn;
-    const int slot = (generic ? 8 : 0) + (pl.block_n / 64 - 1) * 2 + (pl.cta_pair ? 1 : 0);
+    const bool split_cluster = cluster_ctas > 1 && !pl.cta_pair;
+    const int slot = (split_cluster ? 16 : 0) + (generic ? 8 : 0) + (pl.block_n / 64 - 1) * 2 + (pl.cta_pair ? 1 : 0);
     std::lock_guard<std::mutex> lock(g_host_mutex);
     if (dev < 0 || dev >= 64 || !opted_in[dev][slot]) {
       err = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1923,9 +2059,9 @@ int launch(KernelFn fn, const b200_fp8_mm_plan& pl, const CUtensorMap& map_a, co
   cfg.dynamicSmemBytes = static_cast<size_t>(pl.smem_bytes);
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[1];
-  if (pl.cta_pair) {
+  if (cluster_ctas > 1) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster_ctas);
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
@@ -2057,7 +2193,7 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
     const int used = kp.full_tiles < units ? kp.full_tiles : units;
     pl.grid = pl.cta_pair ? 2 * used : used;
   }
-  return launch(fn, pl, map_a, map_b, map_c, kp, stream);
+  return launch(fn, pl, pl.cta_pair ? 2 : 1, map_a, map_b, map_c, kp, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -2130,8 +2266,8 @@ int b200_fp8_mm_static_scratch(const void* a, const void* b, const float* a_scal
   const int sm_count = device_sm_count();
   if (sm_count <= 0) return B200_FP8_MM_ERR_DRIVER;
   b200_fp8_mm_plan pl;
-  choose_plan(M, N, K, sm_count, nullptr, &pl);
-  const size_t need = plan_workspace_bytes(pl);
+  size_t need = 0;
+  choose_plan(M, N, K, sm_count, nullptr, &pl, &need);
   if (need > kStaticScratchBytes) return B200_FP8_MM_ERR_SCRATCH_LIMIT;
   void* scratch = nullptr;
   const int rc = static_scratch_address(&scratch);  // first call on a device looks the address up
@@ -2182,12 +2318,15 @@ size_t b200_fp8_mm_workspace_bytes(int M, int N, int K) {
   // Covers both the plan for K-major operands and the one for MN-major operands (no CTA pairs).
   b200_fp8_mm_plan pl, single;
   const int sms = sm_count_for_sizing();
-  choose_plan(M, N, K, sms, nullptr, &pl);
+  size_t need = 0, need2 = 0;
+  choose_plan(M, N, K, sms, nullptr, &pl, &need);
   memset(&single, 0, sizeof(single));
   single.cta_pair = -1;
   b200_fp8_mm_plan pl2;
-  choose_plan(M, N, K, sms, &single, &pl2);
-  size_t need = plan_workspace_bytes(pl);
+  choose_plan(M, N, K, sms, &single, &pl2, &need2);
+  if (need2 > need) need = need2;
+  // (a plan that runs as clusters needs none of this, but its size as a split plan is covered all the same)
+  if (plan_workspace_bytes(pl) > need) need = plan_workspace_bytes(pl);
   if (plan_workspace_bytes(pl2) > need) need = plan_workspace_bytes(pl2);
   return ((need + 255) / 256) * 256;
 }
