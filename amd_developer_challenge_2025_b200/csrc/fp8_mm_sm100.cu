@@ -36,7 +36,7 @@
 // Grouped form (one launch for G independent problems of the same N and K, e.g. the experts of an MoE layer):
 // a, b, the scales and c carry a leading group dimension, the work list runs over (group, tile), the tensor
 // maps are three-dimensional, and an optional device array gives the number of valid rows per group
-// (tiles past it are skipped by every role, rows past it are never written).
+// (tiles past it are not in the work list, rows past it are never written).
 // With PAIR, two CTAs of a cluster share one 256-row tile: each loads its own 128 rows of A and
 // half of the B rows, the leader CTA issues tcgen05.mma.cta_group::2 for both, and each CTA
 // promotes and stores its own 128 rows. No TMA load uses cluster multicast.
@@ -87,8 +87,8 @@ struct KernelParams {
   int full_tiles;  // tiles [0, full_tiles) run unsplit; the rest are split split_k ways along K
   int raster_group;
   // Reciprocals for decode_work's divisions (see div_small): 1 / (raster_group * tiles_n), 1 / raster_group,
-  // 1 / (rows of the last, shorter raster group), 1 / split_k, 1 / (tiles_m * tiles_n).
-  float rcp_per_group, rcp_raster, rcp_raster_last, rcp_split, rcp_per_problem;
+  // 1 / (rows of the last, shorter raster group), 1 / split_k.
+  float rcp_per_group, rcp_raster, rcp_raster_last, rcp_split;
   int b_scale_rows;
   int vec_store;  // 1 when c, ldc and N allow 16-byte stores
   int stages;
@@ -550,8 +550,14 @@ struct TileCfg {
 struct WorkItem {
   int m0, n0, tile, split, nsplit, kb_begin, kb_end;
   int group;    // 0 unless grouped
-  int m_limit;  // rows [0, m_limit) of the group exist; a tile with m0 >= m_limit is skipped by every role
-  bool skip;
+  int m_limit;  // rows [0, m_limit) of the group exist
+  bool done;    // past the end of the work list (grouped launches; the others know their extent beforehand)
+};
+
+// Where a role stands in a grouped launch's work list: the tiles of groups before `group` take indices [0, base).
+// A role's work indices only grow, so it moves through the groups once per launch.
+struct GroupCursor {
+  int group, base;
 };
 
 // n / d for 0 <= n < 2^22 and d >= 1, with rcp = 1.0f / d: the float quotient is off by at most one, which the
@@ -572,10 +578,16 @@ constexpr int kDivSmallLimit = 1 << 22;
 
 // Work item w -> tile and K range. Tiles are walked in groups of raster_group tile rows, column
 // by column inside a group, so that the CTAs running at one time share A and B tiles in L2.
+//
+// A grouped launch lists only tiles that hold rows: group after group, ceil(valid rows / tile rows) tile rows each, so
+// the row counts (device memory, unknown to the host) decide how many items there are and every CTA gets an equal
+// share of them. With the empty tiles listed and skipped, the CTAs' shares of real ones differed by up to one in
+// three (8 x 1024 x 2048 x 7168 with loads of 1/8 .. 8/8: 160 real tiles of 256 on 74 pairs, four for some and one for others).
 template <bool GENERIC>
-__device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, int tile_m, int block_n) {
+__device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, int tile_m, int block_n, GroupCursor& cur) {
   WorkItem it;
   int t;
+  it.done = false;
   if (w < p.full_tiles) {
     t = w;
     it.split = 0;
@@ -589,27 +601,41 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
     it.split = r - q * p.split_k;
     it.nsplit = p.split_k;
   }
-  const bool small = t < kDivSmallLimit;
+  bool small = t < kDivSmallLimit;
   it.tile = t;
   it.group = 0;
   it.m_limit = p.M;
+  int tiles_m = p.tiles_m;
   if (GENERIC && p.groups > 0) {
-    const int per_problem = p.tiles_m * p.tiles_n;
-    it.group = small ? div_small(t, per_problem, p.rcp_per_problem) : t / per_problem;
-    t -= it.group * per_problem;
-    if (p.m_valid != nullptr) it.m_limit = max(0, min(p.M, __ldg(p.m_valid + it.group)));
+    while (true) {
+      if (p.m_valid != nullptr) {
+        it.m_limit = max(0, min(p.M, __ldg(p.m_valid + cur.group)));
+        tiles_m = (it.m_limit + tile_m - 1) / tile_m;
+      }
+      const int tiles = tiles_m * p.tiles_n;
+      if (w - cur.base < tiles) break;
+      cur.base += tiles;
+      if (++cur.group == p.groups) {
+        it.done = true;
+        return it;
+      }
+    }
+    it.group = cur.group;
+    t = w - cur.base;
+    small = t < kDivSmallLimit;
   }
   const int per_group = p.raster_group * p.tiles_n;
   const int group = small ? div_small(t, per_group, p.rcp_per_group) : t / per_group;
   const int first_m = group * p.raster_group;
-  const bool whole = first_m + p.raster_group <= p.tiles_m;
-  const int gsize = whole ? p.raster_group : p.tiles_m - first_m;
+  const bool whole = first_m + p.raster_group <= tiles_m;
+  const int gsize = whole ? p.raster_group : tiles_m - first_m;
   const int within = t - group * per_group;
-  const int tn = small ? div_small(within, gsize, whole ? p.rcp_raster : p.rcp_raster_last) : within / gsize;
+  float rcp_gsize = whole ? p.rcp_raster : p.rcp_raster_last;
+  if (GENERIC && p.groups > 0 && !whole) rcp_gsize = __frcp_rn(static_cast<float>(gsize));  // a group's own last rows
+  const int tn = small ? div_small(within, gsize, rcp_gsize) : within / gsize;
   const int tm = first_m + (within - tn * gsize);
   it.m0 = tm * tile_m;
   it.n0 = tn * block_n;
-  it.skip = GENERIC && it.m0 >= it.m_limit;
   if (it.nsplit == 1) {
     it.kb_begin = 0;
     it.kb_end = p.kblocks;
@@ -705,7 +731,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 
   // The extent of the work list (kept out of registers across the role split for the same reason).
   auto work_total = [&]() {
-    const int all_tiles = p.tiles_m * p.tiles_n * ((GENERIC && p.groups > 0) ? p.groups : 1);
+    if (GENERIC && p.groups > 0) return p.full_tiles;  // the most there can be; see WorkItem::done
+    const int all_tiles = p.tiles_m * p.tiles_n;
     return p.full_tiles + (all_tiles - p.full_tiles) * p.split_k;
   };
   auto work_begin = [&]() { return PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x); };
@@ -720,9 +747,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
+        GroupCursor cursor{0, 0};
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
-          const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN);
-          if (it.skip) continue;
+          const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
+          if (GENERIC && it.done) break;
           const int a_row = it.m0 + static_cast<int>(cta_rank) * kBlockM;
           const int b_row = it.n0 + static_cast<int>(cta_rank) * (PAIR ? Cfg::kRowsB : 0);
           for (int kb = it.kb_begin; kb < it.kb_end; ++kb) {
@@ -806,9 +834,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         uint32_t my_phase = (me / stages) & 1u;
         int first = me;  // offset of this issuer's next K block from the start of the next tile
         bool ok = true;
+        GroupCursor cursor{0, 0};
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
-          const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN);
-          if (it.skip) continue;
+          const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
+          if (GENERIC && it.done) break;
           int kb = it.kb_begin + first;
           for (; kb < it.kb_end; kb += step) {
             const uint32_t sa = smem_u32(ring + my_stage * Cfg::kStageBytes);
@@ -849,9 +878,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       int slot = 0;
       uint32_t sphase = 0;
       bool ok = true;
+      GroupCursor cursor{0, 0};
       for (int w = work_begin(); w < total_work && ok; w += work_step) {
-        const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN);
-        if (it.skip) continue;
+        const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
+        if (GENERIC && it.done) break;
         const int row0 = it.m0 + static_cast<int>(cta_rank) * kBlockM;
         const float* a_base = p.a_scale + static_cast<long long>(it.group) * p.sa_g;
         const float* a_src[4];
@@ -937,9 +967,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     // warp then stops waiting, fetching and storing but still walks the remaining tiles and takes part in
     // every named barrier of their epilogues, so that warps which have not noticed yet are never left alone
     // at a barrier; they notice at their next wait.
+    GroupCursor cursor{0, 0};
     for (int w = work_begin(); w < total_work; w += work_step) {
-      const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN);
-      if (it.skip) continue;
+      const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
+      if (GENERIC && it.done) break;
       const int row = it.m0 + static_cast<int>(cta_rank) * kBlockM + row_in_tile;
       // Index of this thread's first b_scale row inside a ring slot (at most 2 rows per 128 columns).
       const int gcol0 = it.n0 + col_base + p.n_phase;
@@ -1312,7 +1343,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     cluster_sync_all();
     if (warp >= 4 && *abort_flag == 0) {
       const int ranges = p.split_k;
-      const WorkItem it = decode_work<GENERIC>(p, static_cast<int>(blockIdx.x), Cfg::kTileM, BN);
+      GroupCursor cursor{0, 0};
+      const WorkItem it = decode_work<GENERIC>(p, static_cast<int>(blockIdx.x), Cfg::kTileM, BN, cursor);
       constexpr int kPieces = BN / 4;  // per row
       const int rows = min(kBlockM, p.M - it.m0);
       const uint32_t base = smem_u32(ring);
@@ -1795,7 +1827,6 @@ void set_decode_reciprocals(KernelParams& kp) {
   kp.rcp_raster = 1.0f / static_cast<float>(kp.raster_group);
   kp.rcp_raster_last = 1.0f / static_cast<float>(last > 0 ? last : kp.raster_group);
   kp.rcp_split = 1.0f / static_cast<float>(kp.split_k > 0 ? kp.split_k : 1);
-  kp.rcp_per_problem = 1.0f / static_cast<float>(kp.tiles_m * kp.tiles_n);
 }
 
 // decode_work forms (split + 1) * kblocks in 32 bits; the selector itself never splits more than 16 ways.
