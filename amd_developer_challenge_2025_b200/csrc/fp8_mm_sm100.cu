@@ -297,6 +297,12 @@ __device__ __forceinline__ void tma_store_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
 }
 
+// Programmatic dependent launch. Waits until the kernels this launch depends on have completed and their writes are
+// visible (returns at once in an ordinary launch) ...
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// ... and lets the next kernel's CTAs be scheduled once every CTA of this grid has come here or has left.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void wg_bar_sync(int wg) {
   asm volatile("bar.sync %0, 128;" ::"r"(2 + wg) : "memory");
 }
@@ -725,6 +731,12 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   __syncthreads();
   if constexpr (PAIR) cluster_sync_all();  // the peer's barriers are initialised before any remote arrive
   tcgen05_fence_after();
+  // Everything above touches this CTA's own shared memory, TMEM and kernel parameters only, so it may run under the
+  // tail of the kernel before this one on the stream (programmatic dependent launch); memory is touched from here on.
+  // The kernel after this one may start its own such part as soon as every CTA of this one is on the device: its CTAs
+  // take the SMs that this kernel's CTAs leave, and wait there.
+  pdl_wait();
+  pdl_launch_dependents();
   // The TMEM base address is read again inside each role instead of being carried across the register
   // re-allocation below: a value that is live in every role at once gets one register for all of them, which
   // the promotion warps' accumulators then push out to local memory for everybody.
@@ -2089,14 +2101,17 @@ int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUte
   cfg.blockDim = dim3(static_cast<unsigned>(128 + 32 * epi_warps_for(pl.block_n)), 1, 1);
   cfg.dynamicSmemBytes = static_cast<size_t>(pl.smem_bytes);
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see pdl_wait() in the kernel
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   if (cluster_ctas > 1) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster_ctas);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(cluster_ctas);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
   }
   err = cudaLaunchKernelEx(&cfg, fn, map_a, map_b, map_c, kp);
   if (err != cudaSuccess) {

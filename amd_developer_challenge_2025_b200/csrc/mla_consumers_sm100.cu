@@ -12,6 +12,11 @@
 
 namespace {
 
+// Programmatic dependent launch: a kernel may begin while the one before it on the stream drains; it waits here before
+// it touches memory, and lets the next one begin once all of its own CTAs have been scheduled.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // bf16 arithmetic as the reference writes it: every operation rounds to bf16 (round to nearest even).
 __device__ __forceinline__ __nv_bfloat16 bf(float v) { return __float2bfloat16_rn(v); }
 __device__ __forceinline__ float fl(__nv_bfloat16 v) { return __bfloat162float(v); }
@@ -52,6 +57,8 @@ __global__ void __launch_bounds__(256) rope_kernel(const __nv_bfloat16* __restri
   const int j = static_cast<int>(pair - static_cast<long long>(i1) * half);
   __nv_bfloat16 c, s;
   rope_angle(pos, i1, j, d2, &c, &s);
+  pdl_wait();
+  pdl_launch_dependents();
   const int r0 = blockIdx.y * rows_per_block;
   const int r1 = min(d0, r0 + rows_per_block);
   const __nv_bfloat16* xp = x + static_cast<long long>(i1) * xs2 + j;
@@ -102,6 +109,8 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8(const __nv_bflo
     rope_rotation(use_tab ? base_tab[j] : rope_base(j, d2), pos, i1, &cos_tab[a], &sin_tab[a]);
   }
   __syncthreads();
+  pdl_wait();  // the angles above depend on the arguments only
+  pdl_launch_dependents();
   const int unit = tid & (units - 1);
   const long long g = first + unit;
   if (g >= total) return;
@@ -191,6 +200,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // it, divides by the sum and writes in place. HBM sees one read and one write of the row.
 __global__ void __launch_bounds__(kSoftmaxThreads) div_softmax_kernel(__nv_bfloat16* qk, int sl, float scale2) {
   __shared__ float scratch[kSoftmaxThreads / 32];
+  pdl_wait();
+  pdl_launch_dependents();
   __nv_bfloat16* row = qk + static_cast<long long>(blockIdx.x) * sl;
   // A row starts on a 2-byte boundary: `head` elements up to the next 16-byte boundary go one by one, then
   // 16-byte pieces, then the rest.
@@ -231,6 +242,25 @@ __global__ void __launch_bounds__(kSoftmaxThreads) div_softmax_kernel(__nv_bfloa
 // Rows of up to kRegRowElems elements (the reference's own limit is 8192): the row is read ONCE, its exponentials
 // stay in registers (as the bf16 values the reference keeps) across the block-wide sum, and the quotients are
 // written back; four independent 16-byte loads per thread are in flight at a time.
+// <<<grid, threads>>> on `stream`, allowed to begin under the kernel before it (see pdl_wait).
+template <typename... Params, typename... Args>
+int launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, void* stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return B200_FP8_MM_ERR_LAUNCH;
+  }
+  return B200_FP8_MM_OK;
+}
+
 constexpr int kRegThreads = 256;
 constexpr int kRegVecs = 4;
 constexpr int kRegRowElems = kRegThreads * 8 * kRegVecs;  // 8192 elements in 16-byte pieces, + up to 14 stragglers
@@ -249,6 +279,8 @@ __device__ __forceinline__ float block_sum_256(float v, float* scratch) {
 
 __global__ void __launch_bounds__(kRegThreads, 8) div_softmax_regs_kernel(__nv_bfloat16* qk, int sl, float scale2) {
   __shared__ float scratch[kRegThreads / 32];
+  pdl_wait();
+  pdl_launch_dependents();
   __nv_bfloat16* row = qk + static_cast<long long>(blockIdx.x) * sl;
   const int head = min(sl, static_cast<int>(((16u - (reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) >> 1));
   const int body = ((sl - head) / 8) * 8;
@@ -331,17 +363,12 @@ int b200_mla_rope(const void* x, void* y, int pos, int d0, int d1, int d2, long 
   const int rows_per_block = static_cast<int>(((d0 + want_y - 1) / want_y + row_step - 1) / row_step * row_step);
   const int blocks_y = static_cast<int>((static_cast<long long>(d0) + rows_per_block - 1) / rows_per_block);
   const dim3 grid(static_cast<unsigned>(blocks_x), static_cast<unsigned>(blocks_y));
-  if (vec8) {
-    rope_kernel_vec8<<<grid, kRopeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), pos, d0, d1, d2, xs1, xs2, ys1, ys2,
-        static_cast<int>(units), rows_per_block);
-  } else {
-    rope_kernel<<<grid, kRopeThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), pos, d0, d1, d2, xs1, xs2, ys1, ys2,
-        rows_per_block);
-  }
-  if (cudaGetLastError() != cudaSuccess) return B200_FP8_MM_ERR_LAUNCH;
-  return B200_FP8_MM_OK;
+  const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
+  __nv_bfloat16* yb = static_cast<__nv_bfloat16*>(y);
+  if (vec8)
+    return launch_pdl(rope_kernel_vec8, grid, kRopeThreads, stream, xb, yb, pos, d0, d1, d2, xs1, xs2, ys1, ys2,
+                      static_cast<int>(units), rows_per_block);
+  return launch_pdl(rope_kernel, grid, kRopeThreads, stream, xb, yb, pos, d0, d1, d2, xs1, xs2, ys1, ys2, rows_per_block);
 }
 
 int b200_mla_div_softmax(void* qk, int bs, int nh, int sl, int dnope, int drope, void* stream) {
@@ -351,15 +378,10 @@ int b200_mla_div_softmax(void* qk, int bs, int nh, int sl, int dnope, int drope,
   if (rows > 0x7fffffffll) return B200_FP8_MM_ERR_SHAPE;
   // exp(v / sqrt(d)) = 2^(v * scale2)
   const float scale2 = 1.4426950408889634f / sqrtf(static_cast<float>(dnope + drope));
-  if (sl <= kRegRowElems) {
-    div_softmax_regs_kernel<<<static_cast<unsigned>(rows), kRegThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(qk), sl, scale2);
-  } else {
-    div_softmax_kernel<<<static_cast<unsigned>(rows), kSoftmaxThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(qk), sl, scale2);
-  }
-  if (cudaGetLastError() != cudaSuccess) return B200_FP8_MM_ERR_LAUNCH;
-  return B200_FP8_MM_OK;
+  __nv_bfloat16* data = static_cast<__nv_bfloat16*>(qk);
+  const dim3 grid(static_cast<unsigned>(rows));
+  if (sl <= kRegRowElems) return launch_pdl(div_softmax_regs_kernel, grid, kRegThreads, stream, data, sl, scale2);
+  return launch_pdl(div_softmax_kernel, grid, kSoftmaxThreads, stream, data, sl, scale2);
 }
 
 }  // extern "C"
