@@ -553,6 +553,8 @@ struct TileCfg {
   static_assert(BN % 64 == 0 && BN >= 64 && BN <= 256, "block_n must be 64, 128, 192 or 256");
 };
 
+enum KernelMode { kPlain = 0, kMnMajor = 1, kGrouped = 2 };
+
 struct WorkItem {
   int m0, n0, tile, split, nsplit, kb_begin, kb_end;
   int group;    // 0 unless grouped
@@ -589,7 +591,7 @@ constexpr int kDivSmallLimit = 1 << 22;
 // the row counts (device memory, unknown to the host) decide how many items there are and every CTA gets an equal
 // share of them. With the empty tiles listed and skipped, the CTAs' shares of real ones differed by up to one in
 // three (8 x 1024 x 2048 x 7168 with loads of 1/8 .. 8/8: 160 real tiles of 256 on 74 pairs, four for some and one for others).
-template <bool GENERIC>
+template <int MODE>
 __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, int tile_m, int block_n, GroupCursor& cur) {
   WorkItem it;
   int t;
@@ -612,7 +614,7 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
   it.group = 0;
   it.m_limit = p.M;
   int tiles_m = p.tiles_m;
-  if (GENERIC && p.groups > 0) {
+  if (MODE == kGrouped) {
     while (true) {
       if (p.m_valid != nullptr) {
         it.m_limit = max(0, min(p.M, __ldg(p.m_valid + cur.group)));
@@ -637,7 +639,7 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
   const int gsize = whole ? p.raster_group : tiles_m - first_m;
   const int within = t - group * per_group;
   float rcp_gsize = whole ? p.rcp_raster : p.rcp_raster_last;
-  if (GENERIC && p.groups > 0 && !whole) rcp_gsize = __frcp_rn(static_cast<float>(gsize));  // a group's own last rows
+  if (MODE == kGrouped && !whole) rcp_gsize = __frcp_rn(static_cast<float>(gsize));  // a group's own last rows
   const int tn = small ? div_small(within, gsize, rcp_gsize) : within / gsize;
   const int tm = first_m + (within - tn * gsize);
   it.m0 = tm * tile_m;
@@ -659,12 +661,13 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
 // The kernel
 // ---------------------------------------------------------------------------------------------
 
-// GENERIC = false is the plain case (K-major a and b, one problem): operand layout and work list are
-// compile-time facts and none of the MN-major / grouped code is in the instruction stream of the
-// single-thread roles, whose per-K-block instruction count is on the critical path of narrow tiles.
+// MODE separates the plain case (K-major a and b, one problem), MN-major operands and grouped launches: operand layout
+// and work list are compile-time facts where they can be, and no code of the others is in the instruction stream of
+// the single-thread roles, whose per-K-block instruction count is on the critical path of narrow tiles, or in the
+// registers of the promotion warps, which the 256-wide tiles fill.
 // CLUSTER: the K ranges of a tile are the CTAs of one thread-block cluster (cluster rank = range, one work item per
 // CTA) and the reduction goes through their shared memory; see the end of the kernel.
-template <int BN, bool PAIR, bool GENERIC, bool CLUSTER = false>
+template <int BN, bool PAIR, int MODE, bool CLUSTER = false>
 __global__ void __launch_bounds__((TileCfg<BN, PAIR>::kThreads), 1)
 fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                           const __grid_constant__ CUtensorMap tmap_c, const KernelParams p) {
@@ -743,7 +746,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 
   // The extent of the work list (kept out of registers across the role split for the same reason).
   auto work_total = [&]() {
-    if (GENERIC && p.groups > 0) return p.full_tiles;  // the most there can be; see WorkItem::done
+    if (MODE == kGrouped) return p.full_tiles;  // the most there can be; see WorkItem::done
     const int all_tiles = p.tiles_m * p.tiles_n;
     return p.full_tiles + (all_tiles - p.full_tiles) * p.split_k;
   };
@@ -761,8 +764,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         bool ok = true;
         GroupCursor cursor{0, 0};
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
-          const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
-          if (GENERIC && it.done) break;
+          const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+          if (MODE == kGrouped && it.done) break;
           const int a_row = it.m0 + static_cast<int>(cta_rank) * kBlockM;
           const int b_row = it.n0 + static_cast<int>(cta_rank) * (PAIR ? Cfg::kRowsB : 0);
           for (int kb = it.kb_begin; kb < it.kb_end; ++kb) {
@@ -770,7 +773,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
               ok = false;
               break;
             }
-            if constexpr (BN == 64 && !PAIR && !GENERIC) {
+            if constexpr (BN == 64 && !PAIR && MODE == kPlain) {
               if (kb == p.selftest_skip_kblock && w == work_begin()) {  // self-test only: this block never arrives
                 if (++stage == stages) {
                   stage = 0;
@@ -792,16 +795,16 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             mbar_expect_tx_cluster(fb, Cfg::kStageBytes);
             const uint32_t sa = smem_u32(ring + stage * Cfg::kStageBytes);
             // K-major: x = byte of K, y = matrix row. MN-major: x = matrix row (a multiple of 64), y = k.
-            if (GENERIC && p.groups > 0) {
+            if (MODE == kGrouped) {
               tma_load_3d<PAIR>(sa, &tmap_a, kb * kBlockK, a_row, it.group, fb);
               tma_load_3d<PAIR>(sa + Cfg::kStageBytesA, &tmap_b, kb * kBlockK, b_row, it.group, fb);
             } else {
-            if (!GENERIC || !p.a_mn) {
+            if (MODE != kMnMajor || !p.a_mn) {
               tma_load_2d<PAIR>(sa, &tmap_a, kb * kBlockK, a_row, fb);
             } else {
               tma_load_2d<PAIR>(sa, &tmap_a, a_row, kb * kBlockK, fb);
             }
-            if (!GENERIC || !p.b_mn) {
+            if (MODE != kMnMajor || !p.b_mn) {
               tma_load_2d<PAIR>(sa + Cfg::kStageBytesA, &tmap_b, kb * kBlockK, b_row, fb);
             } else {
               for (int i = 0; i < p.b_boxes; ++i)
@@ -831,10 +834,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       // thread roughly 100 clocks), more than the tensor pipe needs for a narrow tile's block.
       if (lane == 0 && cta_rank == 0 && warp - 1 < p.issuers) {
         constexpr uint32_t kHiK = (1024u >> 4) | (1u << 14) | (2u << 29);  // K-major, 128-byte swizzle
-        const uint32_t idesc = make_idesc(Cfg::kTileM, BN) | (GENERIC ? p.idesc_major : 0u);
-        const uint32_t a_hi = GENERIC ? p.a_desc_hi : kHiK, b_hi = GENERIC ? p.b_desc_hi : kHiK;
-        const uint32_t a_kstep = GENERIC ? p.a_kstep : 2u, b_kstep = GENERIC ? p.b_kstep : 2u;
-        const uint32_t a_lo_bits = GENERIC ? p.a_desc_lo : (1u << 16), b_lo_bits = GENERIC ? p.b_desc_lo : (1u << 16);
+        const uint32_t idesc = make_idesc(Cfg::kTileM, BN) | (MODE == kMnMajor ? p.idesc_major : 0u);
+        const uint32_t a_hi = MODE == kMnMajor ? p.a_desc_hi : kHiK, b_hi = MODE == kMnMajor ? p.b_desc_hi : kHiK;
+        const uint32_t a_kstep = MODE == kMnMajor ? p.a_kstep : 2u, b_kstep = MODE == kMnMajor ? p.b_kstep : 2u;
+        const uint32_t a_lo_bits = MODE == kMnMajor ? p.a_desc_lo : (1u << 16), b_lo_bits = MODE == kMnMajor ? p.b_desc_lo : (1u << 16);
         const int me = warp - 1;
         const int total_work = work_total(), work_step = work_stride();
         const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_base_slot);
@@ -848,8 +851,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         bool ok = true;
         GroupCursor cursor{0, 0};
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
-          const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
-          if (GENERIC && it.done) break;
+          const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+          if (MODE == kGrouped && it.done) break;
           int kb = it.kb_begin + first;
           for (; kb < it.kb_end; kb += step) {
             const uint32_t sa = smem_u32(ring + my_stage * Cfg::kStageBytes);
@@ -892,8 +895,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       bool ok = true;
       GroupCursor cursor{0, 0};
       for (int w = work_begin(); w < total_work && ok; w += work_step) {
-        const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
-        if (GENERIC && it.done) break;
+        const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+        if (MODE == kGrouped && it.done) break;
         const int row0 = it.m0 + static_cast<int>(cta_rank) * kBlockM;
         const float* a_base = p.a_scale + static_cast<long long>(it.group) * p.sa_g;
         const float* a_src[4];
@@ -981,8 +984,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     // at a barrier; they notice at their next wait.
     GroupCursor cursor{0, 0};
     for (int w = work_begin(); w < total_work; w += work_step) {
-      const WorkItem it = decode_work<GENERIC>(p, w, Cfg::kTileM, BN, cursor);
-      if (GENERIC && it.done) break;
+      const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+      if (MODE == kGrouped && it.done) break;
       const int row = it.m0 + static_cast<int>(cta_rank) * kBlockM + row_in_tile;
       // Index of this thread's first b_scale row inside a ring slot (at most 2 rows per 128 columns).
       const int gcol0 = it.n0 + col_base + p.n_phase;
@@ -1191,7 +1194,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       }
       // The TMA store clips at the tensor's edges only: a tile that a group's row count cuts short goes out
       // through the guarded plain stores instead.
-      const bool tma_rows_ok = !GENERIC || (it.m_limit == p.M) || (it.m0 + Cfg::kTileM <= it.m_limit);
+      const bool tma_rows_ok = MODE != kGrouped || (it.m_limit == p.M) || (it.m0 + Cfg::kTileM <= it.m_limit);
       if (do_store && p.store_bufs > 0 && tma_rows_ok) {
         // bf16 tile -> swizzled staging -> TMA store, 32 columns at a time per warpgroup. The
         // 16-byte piece q of row r sits at r*64 + ((q ^ ((r >> 1) & 3)) * 16) (SWIZZLE_64B), which
@@ -1220,7 +1223,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
 #ifdef FP8MM_X_NOSTOREISSUE
           return;
 #endif
-          if (GENERIC && p.groups > 0) {
+          if (MODE == kGrouped) {
             tma_store_3d(&tmap_c, smem_u32(my_stage + bufi * kStoreBufBytes), col0 + ch * kStoreBoxCols,
                          it.m0 + static_cast<int>(cta_rank) * kBlockM, it.group);
           } else {
@@ -1270,7 +1273,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         // row count cuts short: the warp stages 32 columns of its own 32 rows in shared memory and writes them out
         // row by row, sixteen lanes to a row with one 4-byte word each. Left to the thread that owns a row, every
         // store instruction touches 32 rows: 1000 x 4099 x 2304 took 53.2 us that way and takes 28.7 us this way.
-        if constexpr (GENERIC) {
+        if constexpr (MODE == kGrouped) {
           // a tile before this one may have left by bulk stores out of the same buffers
           if (lane == 0) tma_store_wait_read<0>();
           wg_bar_sync(half);
@@ -1356,7 +1359,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     if (warp >= 4 && *abort_flag == 0) {
       const int ranges = p.split_k;
       GroupCursor cursor{0, 0};
-      const WorkItem it = decode_work<GENERIC>(p, static_cast<int>(blockIdx.x), Cfg::kTileM, BN, cursor);
+      const WorkItem it = decode_work<MODE>(p, static_cast<int>(blockIdx.x), Cfg::kTileM, BN, cursor);
       constexpr int kPieces = BN / 4;  // per row
       const int rows = min(kBlockM, p.M - it.m0);
       const uint32_t base = smem_u32(ring);
@@ -1858,34 +1861,40 @@ bool plan_is_supported(const b200_fp8_mm_plan& pl, int kblocks) {
 
 typedef void (*KernelFn)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const KernelParams);
 
-// generic: MN-major operands or a grouped launch (CTA pairs at the 192- and 256-wide tiles only).
-KernelFn kernel_for(int block_n, int pair, bool generic, bool cluster = false) {
-  if (cluster) {
-    if (block_n == 64) return generic ? fp8_mm_blockscaled_kernel<64, false, true, true> : fp8_mm_blockscaled_kernel<64, false, false, true>;
-    if (block_n == 128) return generic ? fp8_mm_blockscaled_kernel<128, false, true, true> : fp8_mm_blockscaled_kernel<128, false, false, true>;
-    return nullptr;
-  }
-  if (generic) {
-    if (pair) {
-      // grouped launches on the two widths where pairs pay
-      if (block_n == 192) return fp8_mm_blockscaled_kernel<192, true, true>;
-      if (block_n == 256) return fp8_mm_blockscaled_kernel<256, true, true>;
-      return nullptr;
-    }
+// The kernel of a tile shape, or null where there is none: CTA pairs take MN-major operands and grouped launches at the
+// two widths where pairs pay, split-K clusters exist for single problems and narrow single-CTA tiles.
+template <int MODE>
+KernelFn kernel_of_mode(int block_n, int pair) {
+  if (pair) {
     switch (block_n) {
-      case 64: return fp8_mm_blockscaled_kernel<64, false, true>;
-      case 128: return fp8_mm_blockscaled_kernel<128, false, true>;
-      case 192: return fp8_mm_blockscaled_kernel<192, false, true>;
-      case 256: return fp8_mm_blockscaled_kernel<256, false, true>;
+      case 64: if constexpr (MODE == kPlain) return fp8_mm_blockscaled_kernel<64, true, MODE>; return nullptr;
+      case 128: if constexpr (MODE == kPlain) return fp8_mm_blockscaled_kernel<128, true, MODE>; return nullptr;
+      case 192: return fp8_mm_blockscaled_kernel<192, true, MODE>;
+      case 256: return fp8_mm_blockscaled_kernel<256, true, MODE>;
       default: return nullptr;
     }
   }
   switch (block_n) {
-    case 64: return pair ? fp8_mm_blockscaled_kernel<64, true, false> : fp8_mm_blockscaled_kernel<64, false, false>;
-    case 128: return pair ? fp8_mm_blockscaled_kernel<128, true, false> : fp8_mm_blockscaled_kernel<128, false, false>;
-    case 192: return pair ? fp8_mm_blockscaled_kernel<192, true, false> : fp8_mm_blockscaled_kernel<192, false, false>;
-    case 256: return pair ? fp8_mm_blockscaled_kernel<256, true, false> : fp8_mm_blockscaled_kernel<256, false, false>;
+    case 64: return fp8_mm_blockscaled_kernel<64, false, MODE>;
+    case 128: return fp8_mm_blockscaled_kernel<128, false, MODE>;
+    case 192: return fp8_mm_blockscaled_kernel<192, false, MODE>;
+    case 256: return fp8_mm_blockscaled_kernel<256, false, MODE>;
     default: return nullptr;
+  }
+}
+
+template <int MODE>
+KernelFn cluster_kernel_of_mode(int block_n) {
+  if (block_n == 64) return fp8_mm_blockscaled_kernel<64, false, MODE, true>;
+  if (block_n == 128) return fp8_mm_blockscaled_kernel<128, false, MODE, true>;
+  return nullptr;
+}
+
+KernelFn kernel_for(int block_n, int pair, KernelMode mode, bool cluster = false) {
+  switch (mode) {
+    case kPlain: return cluster ? cluster_kernel_of_mode<kPlain>(block_n) : kernel_of_mode<kPlain>(block_n, pair);
+    case kMnMajor: return cluster ? cluster_kernel_of_mode<kMnMajor>(block_n) : kernel_of_mode<kMnMajor>(block_n, pair);
+    default: return cluster ? nullptr : kernel_of_mode<kGrouped>(block_n, pair);
   }
 }
 
@@ -1957,13 +1966,14 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   const int sm_count = device_sm_count();
   if (sm_count <= 0) return B200_FP8_MM_ERR_DRIVER;
 
-  // MN-major operands run the GENERIC kernels, which exist for CTA pairs at the 192- and 256-wide tiles. An
+  // MN-major operands run kernels of their own, which exist for CTA pairs at the 192- and 256-wide tiles. An
   // MN-major b needs the CTA's half of the tile's columns to be whole 64-byte boxes, i.e. the 256-wide pair
   // (128 columns per CTA). Where the chosen pair plan has no such kernel, single CTAs are planned instead.
   const bool generic = a_mn || b_mn;
+  const KernelMode mode = generic ? kMnMajor : kPlain;
   auto pair_plan_runs = [&](const b200_fp8_mm_plan& q) {
     if (!generic || !q.cta_pair) return true;
-    if (kernel_for(q.block_n, 1, true) == nullptr) return false;
+    if (kernel_for(q.block_n, 1, mode) == nullptr) return false;
     return !b_mn || ((q.block_n / 2) % 64) == 0;
   };
   const b200_fp8_mm_plan* forced = forced_in;
@@ -1990,7 +2000,7 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
 
   const bool cluster = runs_as_cluster(pl, sm_count);
   if (cluster) pl.grid = pl.tiles * pl.split_k;
-  KernelFn fn = kernel_for(pl.block_n, pl.cta_pair, generic, cluster);
+  KernelFn fn = kernel_for(pl.block_n, pl.cta_pair, mode, cluster);
   if (fn == nullptr) return B200_FP8_MM_ERR_PLAN;
 
   CUtensorMap map_a, map_b, map_c;
@@ -2078,12 +2088,12 @@ int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUte
   // Opt every kernel in to the full 227 KiB of dynamic shared memory once per device.
   cudaError_t err = cudaSuccess;
   {
-    static unsigned char opted_in[64][32] = {};
+    static unsigned char opted_in[64][48] = {};
     int dev = 0;
     (void)cudaGetDevice(&dev);
-    const bool generic = kp.groups > 0 || kp.a_mn || kp.b_mn;
+    const int mode = kp.groups > 0 ? kGrouped : ((kp.a_mn || kp.b_mn) ? kMnMajor : kPlain);
     const bool split_cluster = cluster_ctas > 1 && !pl.cta_pair;
-    const int slot = (split_cluster ? 16 : 0) + (generic ? 8 : 0) + (pl.block_n / 64 - 1) * 2 + (pl.cta_pair ? 1 : 0);
+    const int slot = (split_cluster ? 24 : 0) + mode * 8 + (pl.block_n / 64 - 1) * 2 + (pl.cta_pair ? 1 : 0);
     std::lock_guard<std::mutex> lock(g_host_mutex);
     if (dev < 0 || dev >= 64 || !opted_in[dev][slot]) {
       err = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2165,7 +2175,7 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   }
   if (!plan_is_supported(pl, K / kBlockK) || pl.split_k != 1) return B200_FP8_MM_ERR_PLAN;
   const int tiles_m = ceil_div(M, pl.cta_pair ? 2 * kBlockM : kBlockM);
-  KernelFn fn = kernel_for(pl.block_n, pl.cta_pair, true);
+  KernelFn fn = kernel_for(pl.block_n, pl.cta_pair, kGrouped);
   if (fn == nullptr) return B200_FP8_MM_ERR_PLAN;
 
   CUtensorMap map_a, map_b, map_c;
