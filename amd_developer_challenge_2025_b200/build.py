@@ -16,6 +16,8 @@ SOURCES = [SRC, os.path.join(HERE, "csrc", "mla_consumers_sm100.cu")]
 HEADERS = [os.path.join(INCLUDE, "b200_fp8_mm.h"), os.path.join(INCLUDE, "b200_mla_consumers.h")]
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libb200fp8mm.so")
+HOST_SRC = os.path.join(HERE, "csrc", "host_calls.cpp")  # the entry points' per-call host work (a CPython module)
+HOST_LIB = os.path.join(LIB_DIR, "_host.so")
 
 
 def _nvcc() -> str:
@@ -23,17 +25,35 @@ def _nvcc() -> str:
     return cand if os.path.exists(cand) else "nvcc"
 
 
+def _outdated(target: str, sources) -> bool:
+    return not os.path.exists(target) or os.path.getmtime(target) < max(os.path.getmtime(p) for p in sources)
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
-        return True
-    newest = max(os.path.getmtime(p) for p in SOURCES + HEADERS)
-    return os.path.getmtime(LIB) < newest
+    return _outdated(LIB, SOURCES + HEADERS) or _outdated(HOST_LIB, [HOST_SRC] + HEADERS)
+
+
+def _build_host() -> None:
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    includes = [INCLUDE, sysconfig.get_paths()["include"], *include_paths("cuda")]
+    subprocess.check_call([
+        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+        f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{p}" for p in includes),
+        HOST_SRC, "-o", HOST_LIB, *(f"-L{p}" for p in library_paths()),
+        "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python",
+    ])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB
     os.makedirs(LIB_DIR, exist_ok=True)
+    if force or _outdated(HOST_LIB, [HOST_SRC] + HEADERS):
+        _build_host()
+    if not force and not _outdated(LIB, SOURCES + HEADERS):
+        return LIB
     cmd = [
         _nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
         "-I", INCLUDE, "-shared", "-Xcompiler", "-fPIC", "-o", LIB, *SOURCES,

@@ -113,12 +113,6 @@ def _check(cond: bool, msg: str):
         raise ValueError(msg)
 
 
-# Argument signatures that already passed validation -> (workspace bytes, C plan or None). A repeat
-# call with the same shapes, strides, dtypes and device skips the checks: the operator is called in
-# tight loops and the kernel for a small problem runs for only a few microseconds.
-_validated: dict[tuple, tuple] = {}
-
-
 def _validate(a, b, a_scale, b_scale, c, n_phase, plan):
     _check(a.is_cuda and b.is_cuda and a_scale.is_cuda and b_scale.is_cuda and c.is_cuda,
            "all five tensors must be CUDA tensors (there is no CPU path)")
@@ -160,18 +154,13 @@ def fp8_mm(a, b, a_scale, b_scale, c, n_phase: int = 0, plan: Plan | None = None
     row inside its 128-row scale block (0 unless b is a column shard of a larger matrix).
     `plan`: force tile parameters (sweeps/tests). `check`: synchronise and raise if a wait
     inside the kernel expired. Asynchronous otherwise, like the reference's launcher."""
+    if plan is None and not check and _lib.host_calls().fp8_mm(a, b, a_scale, b_scale, c, n_phase, _workspaces,
+                                                               _status):
+        return c
+    # Not the plain case, or a call that will be refused: the same checks here, with their errors.
     lib = _lib.load()
+    nbytes, cplan = _validate(a, b, a_scale, b_scale, c, n_phase, plan)
     sa, sb, sas, sbs, sc = a.stride(), b.stride(), a_scale.stride(), b_scale.stride(), c.stride()
-    key = (a.shape, b.shape, a_scale.shape, b_scale.shape, c.shape, sa, sb, sas, sbs, sc,
-           a.dtype, b.dtype, a_scale.dtype, b_scale.dtype, c.dtype,
-           a.device, b.device, a_scale.device, b_scale.device, c.device, n_phase, plan)
-    cached = _validated.get(key)
-    if cached is None:
-        cached = _validate(a, b, a_scale, b_scale, c, n_phase, plan)
-        if len(_validated) > 4096:
-            _validated.clear()
-        _validated[key] = cached
-    nbytes, cplan = cached
     m, k = a.shape
     n = b.shape[0]
     dev = a.device
@@ -232,6 +221,8 @@ def fp8_mm_grouped(a, b, a_scale, b_scale, c, m_valid=None, plan: Plan | None = 
     `torch.bmm` (2-amd-moe/amd-moe-submission.py:604-611). a_scale: fp32 [G, M, K/128]; b_scale: fp32
     [G, ceil(N/128), K/128]; any strides for the scales, K contiguous for a and b. `m_valid`: optional
     int32 CUDA tensor [G]; rows at or past m_valid[g] of group g are neither computed nor written."""
+    if plan is None and not check and _lib.host_calls().fp8_mm_grouped(a, b, a_scale, b_scale, c, m_valid, _status):
+        return c
     lib = _lib.load()
     _check(all(t.is_cuda for t in (a, b, a_scale, b_scale, c)), "all tensors must be CUDA tensors (there is no CPU path)")
     _check(a.dtype == torch.float8_e4m3fn and b.dtype == torch.float8_e4m3fn, "a and b must be float8_e4m3fn")

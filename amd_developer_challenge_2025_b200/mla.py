@@ -17,6 +17,9 @@ def mla_decode(x, y, pos: int, xoff: int, yoff: int, d0: int, d1: int, d2: int, 
     """Rotary position embedding, the reference's `module.mla_decode`: reads the bf16 elements
     x.data_ptr() + xoff + i0*xs1 + i1*xs2 + j and writes the rotated values to y at yoff + i0*ys1 + i1*ys2 + j
     (i0 < d0, i1 < d1, j < d2; row i1 has position pos + i1). y may be x. Runs on the current stream."""
+    if _lib.host_calls().mla_decode(x, y, pos, xoff, yoff, d0, d1, d2, xs1, xs2, ys1, ys2):
+        return y
+    # Not the plain case, or a call that will be refused: the same checks here, with their errors.
     _check(x.is_cuda and y.is_cuda and x.device == y.device, "x and y must be CUDA tensors on one device")
     _check(x.dtype == torch.bfloat16 and y.dtype == torch.bfloat16, "x and y must be bfloat16")
     _check(d0 > 0 and d1 > 0 and d2 > 0 and d2 % 2 == 0, "d0, d1, d2 must be positive and d2 even")
@@ -36,6 +39,8 @@ def mla_decode(x, y, pos: int, xoff: int, yoff: int, d0: int, d1: int, d2: int, 
 def div_softmax(qk, bs: int, nh: int, sl: int, dnope: int, drope: int):
     """In-place softmax(qk / sqrt(dnope + drope)) over the last dimension of the contiguous bf16 tensor
     qk [bs, nh, sl], the reference's `module.div_softmax`. Runs on the current stream."""
+    if _lib.host_calls().div_softmax(qk, bs, nh, sl, dnope, drope):
+        return qk
     _check(qk.is_cuda and qk.dtype == torch.bfloat16 and qk.is_contiguous(), "qk must be a contiguous bfloat16 CUDA tensor")
     _check(qk.numel() == bs * nh * sl and bs > 0 and nh > 0 and sl > 0, "qk must hold bs * nh * sl elements")
     with torch.cuda.device(qk.device):
