@@ -95,7 +95,7 @@ struct KernelParams {
   int tmem_bufs;  // TMEM partial buffers in use: divides stages, at most TileCfg::kTmemBufs
   int issuers;     // MMA-issuing threads in use: 1 or 2
   int store_bufs;  // staging buffers per promotion warpgroup for the TMA store of c: 0 (plain stores), 1 .. 4
-  int row_stage_bufs;  // the same buffers when tiles leave row by row instead (store_bufs as planned); 0: no staging
+  int row_stage_bufs;  // the same buffers where the TMA store cannot address c and tiles leave row by row; 0: no staging
   // Operand layout, as the values the producer and the MMA threads need (see OperandLayout below).
   int a_mn, b_mn;            // 1: the operand is MN-major in global and shared memory
   int b_boxes;               // TMA boxes per stage of b (1 when K-major)
@@ -1269,15 +1269,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           }
         }
       } else if (do_store && p.row_stage_bufs > 0) {
-        // Rows of c that the TMA store cannot address (base or pitch not 16-byte aligned), or a tile that a group's
-        // row count cuts short: the warp stages 32 columns of its own 32 rows in shared memory and writes them out
-        // row by row, sixteen lanes to a row with one 4-byte word each. Left to the thread that owns a row, every
-        // store instruction touches 32 rows: 1000 x 4099 x 2304 took 53.2 us that way and takes 28.7 us this way.
-        if constexpr (MODE == kGrouped) {
-          // a tile before this one may have left by bulk stores out of the same buffers
-          if (lane == 0) tma_store_wait_read<0>();
-          wg_bar_sync(half);
-        }
+        // Rows of c whose base or pitch is not 16-byte aligned: the warp stages 32 columns of its own 32 rows in shared
+        // memory and writes them out row by row, sixteen lanes to a row with one 4-byte word each. Left to the thread
+        // that owns a row, every store instruction touches 32 rows: 1000 x 4099 x 2304 took 53.2 us that way and takes
+        // 24.6 us this way.
         constexpr int kBoxes = Cfg::kColsPerThread / kStoreBoxCols;
         uint8_t* warp_stage = staging + half * p.row_stage_bufs * kStoreBufBytes + quarter * (32 * 64);
         const int m_warp = row - lane;  // first row of this warp
@@ -1299,26 +1294,28 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           }
           __syncwarp();
           const int cols = min(kStoreBoxCols, p.N - (col0 + ch * kStoreBoxCols));  // columns of this box that exist
-          for (int r = sub; r < rows; r += 2) {
+#pragma unroll 4
+          for (int i = 0; i < 16; ++i) {
+            const int r = 2 * i + sub;
             __nv_bfloat16* dst = cwarp + static_cast<long long>(r) * p.ldc + col0 + ch * kStoreBoxCols;
-            const uint8_t* src = warp_stage + r * 64;
-            const int sw = (r >> 1) & 3;
-            auto at = [&](int e) -> uint32_t {  // bf16 element e of the staged row
-              return *reinterpret_cast<const unsigned short*>(src + ((((e >> 3) ^ sw) << 4) | ((e & 7) << 1)));
-            };
-            // Word w of the row holds elements 2w - odd and 2w - odd + 1, where odd = 1 when the row starts between
-            // two words; element -1 does not exist, and element 31 is then a half word of its own.
-            const int odd = static_cast<int>((reinterpret_cast<uintptr_t>(dst) >> 1) & 1u);
-            const int e0 = 2 * word - odd;
-            const uint32_t lo = e0 >= 0 ? at(e0) : 0u, hi = at(e0 + 1);
-            if (e0 >= 0 && e0 + 1 < cols) {
-              *reinterpret_cast<uint32_t*>(dst + e0) = lo | (hi << 16);
-            } else {
-              if (e0 >= 0 && e0 < cols) *reinterpret_cast<unsigned short*>(dst + e0) = static_cast<unsigned short>(lo);
-              if (e0 < 0 && cols > 0) *reinterpret_cast<unsigned short*>(dst) = static_cast<unsigned short>(hi);
+            // Word w of the staged row (elements 2w, 2w + 1). A row that starts between two words of global memory
+            // (odd) is written as elements 2w - 1 and 2w, the former from the lane before; element 31 is then left over.
+            const uint32_t cur = *reinterpret_cast<const uint32_t*>(
+                warp_stage + r * 64 + ((((word >> 2) ^ ((r >> 1) & 3)) << 4) | ((word & 3) << 2)));
+            const uint32_t before = __shfl_up_sync(0xffffffffu, cur, 1, 16);
+            const bool odd = ((reinterpret_cast<uintptr_t>(dst) >> 1) & 1u) != 0;
+            const int e0 = 2 * word - (odd ? 1 : 0);
+            const uint32_t two = odd ? __funnelshift_r(before, cur, 16) : cur;
+            if (r < rows) {
+              if (e0 >= 0 && e0 + 1 < cols) {
+                *reinterpret_cast<uint32_t*>(dst + e0) = two;
+              } else {
+                if (e0 >= 0 && e0 < cols) *reinterpret_cast<unsigned short*>(dst + e0) = static_cast<unsigned short>(two);
+                if (e0 < 0 && cols > 0) *reinterpret_cast<unsigned short*>(dst) = static_cast<unsigned short>(cur);
+              }
+              if (odd && word == 15 && cols == kStoreBoxCols)
+                *reinterpret_cast<unsigned short*>(dst + 31) = static_cast<unsigned short>(cur >> 16);
             }
-            if (odd && word == 15 && cols == kStoreBoxCols)
-              *reinterpret_cast<unsigned short*>(dst + 31) = static_cast<unsigned short>(at(31));
           }
           __syncwarp();
         }
@@ -2042,7 +2039,7 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   kp.stages = pl.stages;
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
   kp.store_bufs = store_bufs;
-  kp.row_stage_bufs = pl.store_bufs;
+  kp.row_stage_bufs = (reinterpret_cast<uintptr_t>(c) % 16) != 0 || (ldc % 8) != 0 ? pl.store_bufs : 0;
   kp.a_mn = a_mn ? 1 : 0;
   kp.b_mn = b_mn ? 1 : 0;
   kp.b_boxes = lb.boxes;
@@ -2214,7 +2211,9 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.stages = pl.stages;
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
   kp.store_bufs = store_bufs;
-  kp.row_stage_bufs = pl.store_bufs;
+  // (a tile that a group's row count cuts short leaves in 16-byte pieces where c allows them: 17 x 340 x 2304 x 384
+  // with uneven loads 23.9 us, staged row by row 32.0)
+  kp.row_stage_bufs = store_bufs == 0 ? pl.store_bufs : 0;
   kp.b_boxes = lb.boxes;
   kp.b_box_cols = lb.box_cols;
   kp.b_box_bytes = lb.box_bytes;
