@@ -92,6 +92,7 @@ struct KernelParams {
   int b_scale_rows;
   int vec_store;  // 1 when c, ldc and N allow 16-byte stores
   int stages;
+  uint32_t stage_tx;  // bytes the copies of one K block bring to this CTA's stage
   int tmem_bufs;  // TMEM partial buffers in use: divides stages, at most TileCfg::kTmemBufs
   int issuers;     // MMA-issuing threads in use: 1 or 2
   int store_bufs;  // staging buffers per promotion warpgroup for the TMA store of c: 0 (plain stores), 1 .. 4
@@ -792,7 +793,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             }
             continue;
 #endif
-            mbar_expect_tx_cluster(fb, Cfg::kStageBytes);
+            mbar_expect_tx_cluster(fb, p.stage_tx);
             const uint32_t sa = smem_u32(ring + stage * Cfg::kStageBytes);
             // K-major: x = byte of K, y = matrix row. MN-major: x = matrix row (a multiple of 64), y = k.
             if (MODE == kGrouped) {
@@ -1594,6 +1595,13 @@ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 // Rows of b per TMA box of one CTA (K-major b): a CTA of a pair loads half of the tile's rows.
 int b_box_rows_for(int block_n, int pair) { return pair ? block_n / 2 : block_n; }
 
+// Rows of a per TMA box (K-major a): the tile's 128, or, where there is but one tile row and it is not full, the rows
+// that exist, in whole swizzle atoms of eight. A box row outside the matrix is no cheaper than one inside: it is filled
+// with zeros at less than the rate of real data (64-wide tiles on 4608 x 7168: one row took 25.7 us with whole boxes
+// where 128 rows took 18.5, and takes 17.6). The rest of the stage holds whatever was there; it only reaches rows of the
+// accumulator that are never read.
+int a_box_rows_for(int M) { return M < kBlockM ? ((M + 7) / 8) * 8 : kBlockM; }
+
 int epi_warps_for(int block_n) {
   (void)block_n;
   return 8;  // keep in step with TileCfg::kEpiWarps
@@ -2011,7 +2019,8 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   }
   const OperandLayout la = operand_layout(a_mn, kBlockM);
   const OperandLayout lb = operand_layout(b_mn, b_box_rows_for(pl.block_n, pl.cta_pair));
-  if (!encode_operand_map(&map_a, a, M, K, lda, la.box_cols, a_mn)) return B200_FP8_MM_ERR_DRIVER;
+  const int a_box = a_mn ? la.box_cols : a_box_rows_for(M);
+  if (!encode_operand_map(&map_a, a, M, K, lda, a_box, a_mn)) return B200_FP8_MM_ERR_DRIVER;
   if (!encode_operand_map(&map_b, b, N, K, ldb, lb.box_cols, b_mn)) return B200_FP8_MM_ERR_DRIVER;
 
   KernelParams kp;
@@ -2037,6 +2046,7 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   kp.full_tiles = pl.full_tiles;
   kp.kblocks = kblocks;
   kp.stages = pl.stages;
+  kp.stage_tx = static_cast<uint32_t>((a_box + b_box_rows_for(pl.block_n, pl.cta_pair)) * kBlockK);
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
   kp.store_bufs = store_bufs;
   kp.row_stage_bufs = (reinterpret_cast<uintptr_t>(c) % 16) != 0 || (ldc % 8) != 0 ? pl.store_bufs : 0;
@@ -2183,7 +2193,8 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   } else {
     memset(&map_c, 0, sizeof(map_c));
   }
-  if (!encode_operand_map_3d(&map_a, a, groups, M, K, lda, a_g, kBlockM)) return B200_FP8_MM_ERR_DRIVER;
+  const int a_box = a_box_rows_for(M);
+  if (!encode_operand_map_3d(&map_a, a, groups, M, K, lda, a_g, a_box)) return B200_FP8_MM_ERR_DRIVER;
   const int b_rows_per_cta = b_box_rows_for(pl.block_n, pl.cta_pair);
   if (!encode_operand_map_3d(&map_b, b, groups, N, K, ldb, b_g, b_rows_per_cta)) return B200_FP8_MM_ERR_DRIVER;
 
@@ -2209,6 +2220,7 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.full_tiles = groups * kp.tiles_m * kp.tiles_n;
   kp.kblocks = K / kBlockK;
   kp.stages = pl.stages;
+  kp.stage_tx = static_cast<uint32_t>((a_box + b_rows_per_cta) * kBlockK);
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
   kp.store_bufs = store_bufs;
   // (a tile that a group's row count cuts short leaves in 16-byte pieces where c allows them: 17 x 340 x 2304 x 384
