@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kSoftmaxThreads) div_softmax_kernel(__nv_bfloa
   }
 }
 
-// Rows of up to kRegRowElems elements (the reference's own limit is 8192): the row is read ONCE, its exponentials
+// Longer rows, up to kRegRowElems elements (the reference's own limit is 8192): the row is read ONCE, its exponentials
 // stay in registers (as the bf16 values the reference keeps) across the block-wide sum, and the quotients are
 // written back; four independent 16-byte loads per thread are in flight at a time.
 // <<<grid, threads>>> on `stream`, allowed to begin under the kernel before it (see pdl_wait).
@@ -327,6 +327,68 @@ __global__ void __launch_bounds__(kRegThreads, 8) div_softmax_regs_kernel(__nv_b
   if (static_cast<int>(threadIdx.x) < rest) row[si] = bf(fl(stray) * inv);
 }
 
+// Short rows: one warp per row, VECS 16-byte pieces per lane, otherwise as the register kernel above. A CTA per row
+// leaves most of its threads without an element and pays a block-wide sum for a few hundred values; here eight rows
+// share a CTA and the sum is five shuffles.
+constexpr int kWarpRowThreads = 256;
+constexpr int kWarpRowMaxVecs = 8;
+constexpr int kWarpRowElems = 32 * 8 * kWarpRowMaxVecs;  // 2048
+
+template <int VECS>
+__global__ void __launch_bounds__(kWarpRowThreads) div_softmax_warp_kernel(__nv_bfloat16* qk, int rows, int sl,
+                                                                          float scale2) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const long long r = static_cast<long long>(blockIdx.x) * (kWarpRowThreads / 32) + (threadIdx.x >> 5);
+  if (r >= rows) return;
+  __nv_bfloat16* row = qk + r * sl;
+  const int head = min(sl, static_cast<int>(((16u - (reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) >> 1));
+  const int body = ((sl - head) / 8) * 8;
+  const int rest = sl - body;  // head + tail elements, at most 14: one per lane
+  __nv_bfloat16* vrow = row + head;
+  uint4 raw[VECS];
+#pragma unroll
+  for (int v = 0; v < VECS; ++v) {
+    const int i = (lane + v * 32) * 8;
+    raw[v] = (i < body) ? *reinterpret_cast<const uint4*>(vrow + i) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  const int si = lane < head ? lane : body + lane;
+  __nv_bfloat16 stray = bf(0.f);
+  float sum = 0.f;
+  if (lane < rest) {
+    const float e = exp2_fast(fl(row[si]) * scale2);
+    sum += e;
+    stray = bf(e);
+  }
+#pragma unroll
+  for (int v = 0; v < VECS; ++v) {
+    if ((lane + v * 32) * 8 < body) {
+      uint32_t* w = reinterpret_cast<uint32_t*>(&raw[v]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float a = exp2_fast(lo_f(w[e]) * scale2), b = exp2_fast(hi_f(w[e]) * scale2);
+        sum += a + b;
+        w[e] = pack_bf16(a, b);  // kept as the bf16 values the reference stores
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  const float inv = 1.0f / sum;
+#pragma unroll
+  for (int v = 0; v < VECS; ++v) {
+    const int i = (lane + v * 32) * 8;
+    if (i < body) {
+      uint32_t* w = reinterpret_cast<uint32_t*>(&raw[v]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = pack_bf16(lo_f(w[e]) * inv, hi_f(w[e]) * inv);
+      *reinterpret_cast<uint4*>(vrow + i) = raw[v];
+    }
+  }
+  if (lane < rest) row[si] = bf(fl(stray) * inv);
+}
+
 }  // namespace
 
 extern "C" {
@@ -379,6 +441,17 @@ int b200_mla_div_softmax(void* qk, int bs, int nh, int sl, int dnope, int drope,
   // exp(v / sqrt(d)) = 2^(v * scale2)
   const float scale2 = 1.4426950408889634f / sqrtf(static_cast<float>(dnope + drope));
   __nv_bfloat16* data = static_cast<__nv_bfloat16*>(qk);
+  // One warp per row where rows are short, or where there are more of them than CTAs on the device at a time: 16384 rows
+  // of 64 elements 4.4 us (one CTA per row 21.4), of 1024 11.9 (26.1), of 2048 22.5 (31.9); but 16 rows of 2048, whose
+  // latency is all that counts, 3.3 us against 1.9.
+  if (sl <= 32 * 16 || (sl <= kWarpRowElems && rows > 148 * 8)) {
+    const dim3 warps(static_cast<unsigned>((rows + kWarpRowThreads / 32 - 1) / (kWarpRowThreads / 32)));
+    const int n = static_cast<int>(rows);
+    if (sl <= 32 * 8) return launch_pdl(div_softmax_warp_kernel<1>, warps, kWarpRowThreads, stream, data, n, sl, scale2);
+    if (sl <= 32 * 16) return launch_pdl(div_softmax_warp_kernel<2>, warps, kWarpRowThreads, stream, data, n, sl, scale2);
+    if (sl <= 32 * 32) return launch_pdl(div_softmax_warp_kernel<4>, warps, kWarpRowThreads, stream, data, n, sl, scale2);
+    return launch_pdl(div_softmax_warp_kernel<8>, warps, kWarpRowThreads, stream, data, n, sl, scale2);
+  }
   const dim3 grid(static_cast<unsigned>(rows));
   if (sl <= kRegRowElems) return launch_pdl(div_softmax_regs_kernel, grid, kRegThreads, stream, data, sl, scale2);
   return launch_pdl(div_softmax_kernel, grid, kSoftmaxThreads, stream, data, sl, scale2);
