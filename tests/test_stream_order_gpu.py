@@ -1,6 +1,8 @@
 """Launches that may begin under the kernel before them still read and write in stream order: chains in which every call
 depends on the one before it, with and without other kernels between, on two streams, and inside a CUDA graph, give the
 bits of the same calls run one at a time."""
+import random
+
 import pytest
 import torch
 
@@ -70,3 +72,35 @@ def test_chain_equals_one_call_at_a_time(m, how):
     check_device_status()
     for g, w in zip(got, want):
         assert torch.equal(g.view(torch.uint8), w.view(torch.uint8))
+
+
+@pytest.mark.parametrize("seed", range(3))
+def test_different_problems_back_to_back(seed):
+    """Neighbouring launches differ in shape, kernel, addresses and tensor maps; nothing waits between them."""
+    rng = random.Random(seed)
+    shapes = [(1, 576, 7168), (300, 2000, 512), (128, 576, 7168), (257, 4099, 384), (2048, 512, 1024), (64, 1536, 2048),
+              (1000, 1000, 640), (16, 128, 128), (600, 600, 3584), (513, 3072, 256)]
+    rng.shuffle(shapes)
+    jobs = []
+    for i, (m, n, k) in enumerate(shapes * 2):
+        g = torch.Generator(device="cuda").manual_seed(100 * seed + i)
+        a, b = (torch.randn(r, k, device="cuda", generator=g).to(torch.float8_e4m3fn) for r in (m, n))
+        a_s, b_s = (0.01 + torch.rand(r, k // 128, device="cuda", generator=g) for r in (m, (n + 127) // 128))
+        if m % 16 == 0 and n % 16 == 0 and i % 2:
+            a, b = (t.t().contiguous().t() for t in (a, b))
+        jobs.append((a, b, a_s, b_s))
+    want = []
+    for (a, b, a_s, b_s) in jobs:
+        c = torch.zeros(a.shape[0], b.shape[0], dtype=torch.bfloat16, device="cuda")
+        pkg.custom_kernel((a, b, a_s, b_s, c))
+        torch.cuda.synchronize()
+        want.append(c)
+    got = [torch.zeros_like(c) for c in want]
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for (a, b, a_s, b_s), c in zip(jobs, got):
+            pkg.custom_kernel((a, b, a_s, b_s, c))
+    torch.cuda.synchronize()
+    check_device_status()
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
