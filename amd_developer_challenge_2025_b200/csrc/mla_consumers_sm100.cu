@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(256) rope_kernel(const __nv_bfloat16* __restri
 
 constexpr int kRopeThreads = 256;
 constexpr int kRopeTable = 256;     // pair indices whose 10000^(-2j/d2) a CTA keeps in shared memory
-constexpr int kRopeWidePairs = 16384;  // from here on a CTA takes kRopeMaxUnits units
-constexpr int kRopeMaxUnits = 256;  // units (position, eight adjacent pair indices) of one CTA
+constexpr int kRopeWidePairs = 16384;  // from here on rope_kernel_vec8_wide
+constexpr int kRopeMaxUnits = 128;  // units (position, eight adjacent pair indices) of one CTA that shares its angles
 
 // The same with eight adjacent pair indices per thread: 16-byte loads and stores. Used when d2/2 is a multiple of 8
 // and every row start is 16-byte aligned (checked by the launcher).
@@ -159,6 +159,80 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8(const __nv_bflo
     for (int u = 0; u < kRowsInFlight; ++u) rotate_store(a[u], b[u], i0 + u * step);
   }
   for (; i0 < r1; i0 += step) {
+    const uint4 a = *reinterpret_cast<const uint4*>(xp + i0 * xs1);
+    const uint4 b = *reinterpret_cast<const uint4*>(xp + i0 * xs1 + half);
+    rotate_store(a, b, i0);
+  }
+}
+
+// The same for many units (the keys of a whole cache) or a single row: one unit per thread, its angles in registers, the
+// rows one after the other, so that the CTAs running together sweep few rows from end to end, which HBM likes best. The
+// keys of 128 rows x 6145 positions: 38.0 us; 44.2 in the kernel above with 256 units, 41 to 45 with 32 to 128.
+__global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8_wide(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* y, int pos,
+                                                        int d0, int d1, int d2, long long xs1, long long xs2,
+                                                        long long ys1, long long ys2, int rows_per_block) {
+  const int half = d2 >> 1;
+  const int groups = half >> 3;  // groups of eight pair indices per position row
+  // 10000^(-2j/d2) depends on j alone: the CTA computes the table once (powf is about half of a thread's angle
+  // arithmetic) when it fits; every thread then needs only a cosf and a sinf per pair index.
+  __shared__ __nv_bfloat16 base_tab[kRopeTable];
+  const bool use_tab = half <= kRopeTable;
+  if (use_tab) {
+    for (int j = threadIdx.x; j < half; j += blockDim.x) base_tab[j] = rope_base(j, d2);
+    __syncthreads();
+  }
+  const long long g = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (g >= static_cast<long long>(d1) * groups) return;
+  const int i1 = static_cast<int>(g / groups);
+  const int j0 = static_cast<int>(g - static_cast<long long>(i1) * groups) * 8;
+  __nv_bfloat16 c[8], s[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    __nv_bfloat16 ce, se;
+    rope_rotation(use_tab ? base_tab[j0 + e] : rope_base(j0 + e, d2), pos, i1, &ce, &se);
+    c[e] = ce;
+    s[e] = se;
+  }
+  pdl_wait();  // the angles above depend on the arguments only
+  pdl_launch_dependents();
+  const int r0 = blockIdx.y * rows_per_block;
+  const int r1 = min(d0, r0 + rows_per_block);
+  const __nv_bfloat16* xp = x + static_cast<long long>(i1) * xs2 + j0;
+  __nv_bfloat16* yp = y + static_cast<long long>(i1) * ys2 + j0;
+  constexpr int kRowsInFlight = 4;  // as above
+  // (packed arithmetic as above)
+  __nv_bfloat162 c2[4], s2[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    c2[e] = __halves2bfloat162(c[2 * e], c[2 * e + 1]);
+    s2[e] = __halves2bfloat162(s[2 * e], s[2 * e + 1]);
+  }
+  auto rotate_store = [&](const uint4& a, const uint4& b, int i0) {
+    const __nv_bfloat162* x1 = reinterpret_cast<const __nv_bfloat162*>(&a);
+    const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&b);
+    uint4 o1, o2;
+    __nv_bfloat162* y1 = reinterpret_cast<__nv_bfloat162*>(&o1);
+    __nv_bfloat162* y2 = reinterpret_cast<__nv_bfloat162*>(&o2);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      y1[e] = __hsub2_rn(__hmul2_rn(x1[e], c2[e]), __hmul2_rn(x2[e], s2[e]));
+      y2[e] = __hadd2_rn(__hmul2_rn(x2[e], c2[e]), __hmul2_rn(x1[e], s2[e]));
+    }
+    *reinterpret_cast<uint4*>(yp + i0 * ys1) = o1;
+    *reinterpret_cast<uint4*>(yp + i0 * ys1 + half) = o2;
+  };
+  int i0 = r0;
+  for (; i0 + kRowsInFlight <= r1; i0 += kRowsInFlight) {
+    uint4 a[kRowsInFlight], b[kRowsInFlight];
+#pragma unroll
+    for (int u = 0; u < kRowsInFlight; ++u) {
+      a[u] = *reinterpret_cast<const uint4*>(xp + (i0 + u) * xs1);
+      b[u] = *reinterpret_cast<const uint4*>(xp + (i0 + u) * xs1 + half);
+    }
+#pragma unroll
+    for (int u = 0; u < kRowsInFlight; ++u) rotate_store(a[u], b[u], i0 + u);
+  }
+  for (; i0 < r1; ++i0) {
     const uint4 a = *reinterpret_cast<const uint4*>(xp + i0 * xs1);
     const uint4 b = *reinterpret_cast<const uint4*>(xp + i0 * xs1 + half);
     rotate_store(a, b, i0);
@@ -401,18 +475,16 @@ int b200_mla_rope(const void* x, void* y, int pos, int d0, int d1, int d2, long 
   const bool vec8 = (half % 8) == 0 && (xs1 % 8) == 0 && (xs2 % 8) == 0 && (ys1 % 8) == 0 && (ys2 % 8) == 0 &&
                     (reinterpret_cast<uintptr_t>(x) % 16) == 0 && (reinterpret_cast<uintptr_t>(y) % 16) == 0;
   const long long pairs = static_cast<long long>(d1) * (vec8 ? half / 8 : half);
-  // Units per CTA of the 16-byte kernel. Many units (the keys of a whole cache): as wide a CTA as there is, so that
-  // the CTAs running together sweep few rows from end to end, which HBM likes best (6145 positions x 128 rows: 256
-  // units 38 us, 32 to 128 units 41 to 45). Fewer: 32, so that there are CTAs for every SM (2049 positions x 32 rows:
-  // 5.2 against 6.1 us). Never more threads for the units than rows leave idle, never fewer units than one per row
-  // slot, and more where the grid would otherwise pass its limit.
+  // Units per CTA of the 16-byte kernels. Many units: one per thread (rope_kernel_vec8_wide). Fewer: 32, so that there
+  // are CTAs for every SM (2049 positions x 32 rows: 5.2 against 6.1 us); no more than there are, and no fewer than leave
+  // every row slot a row, up to one per thread again.
   long long units = kRopeThreads;
   if (vec8 && pairs < kRopeWidePairs) {
     units = 1;
     while (units < pairs && units < 32) units *= 2;
-    while (units < kRopeMaxUnits && kRopeThreads / units > d0) units *= 2;
+    while (units < kRopeThreads && kRopeThreads / units > d0) units *= 2;
   }
-  const int ctas_per_sm = (vec8 && units < kRopeMaxUnits) ? 4 : 2;
+  const int ctas_per_sm = (vec8 && units < kRopeThreads) ? 4 : 2;
   const long long blocks_x = (pairs + units - 1) / units;
   if (blocks_x > 0x7fffffffll) return B200_FP8_MM_ERR_SHAPE;
   // Rows per CTA: CTAs for every SM a few times over (each evaluates its units' angles once).
@@ -427,6 +499,9 @@ int b200_mla_rope(const void* x, void* y, int pos, int d0, int d1, int d2, long 
   const dim3 grid(static_cast<unsigned>(blocks_x), static_cast<unsigned>(blocks_y));
   const __nv_bfloat16* xb = static_cast<const __nv_bfloat16*>(x);
   __nv_bfloat16* yb = static_cast<__nv_bfloat16*>(y);
+  if (vec8 && units == kRopeThreads)
+    return launch_pdl(rope_kernel_vec8_wide, grid, kRopeThreads, stream, xb, yb, pos, d0, d1, d2, xs1, xs2, ys1, ys2,
+                      rows_per_block);
   if (vec8)
     return launch_pdl(rope_kernel_vec8, grid, kRopeThreads, stream, xb, yb, pos, d0, d1, d2, xs1, xs2, ys1, ys2,
                       static_cast<int>(units), rows_per_block);
