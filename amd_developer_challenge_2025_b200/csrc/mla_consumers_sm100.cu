@@ -16,6 +16,9 @@ namespace {
 // it touches memory, and lets the next one begin once all of its own CTAs have been scheduled.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// No pointer in this file is `const __restrict__`, and no load goes by __ldg: those are read-only loads, which the compiler
+// may move above pdl_wait() and which may be answered from a line that the kernel before this one has replaced since. y may
+// also be x.
 
 // bf16 arithmetic as the reference writes it: every operation rounds to bf16 (round to nearest even).
 __device__ __forceinline__ __nv_bfloat16 bf(float v) { return __float2bfloat16_rn(v); }
@@ -47,7 +50,7 @@ __device__ __forceinline__ void rope_angle(int pos, int i1, int j, int d2, __nv_
 // One thread owns one (i1, j) pair and a share of the d0 rows: the angle is computed once and reused for
 // every row. Consecutive threads take consecutive j, so a warp reads two runs of 64 contiguous bytes per row.
 // grid.x covers the d1 * d2/2 pairs, grid.y cuts d0 so that small d1 (the query: one position) still fills the GPU.
-__global__ void __launch_bounds__(256) rope_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* y, int pos,
+__global__ void __launch_bounds__(256) rope_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, int pos,
                                                    int d0, int d1, int d2, long long xs1, long long xs2,
                                                    long long ys1, long long ys2, int rows_per_block) {
   const int half = d2 >> 1;
@@ -63,12 +66,25 @@ __global__ void __launch_bounds__(256) rope_kernel(const __nv_bfloat16* __restri
   const int r1 = min(d0, r0 + rows_per_block);
   const __nv_bfloat16* xp = x + static_cast<long long>(i1) * xs2 + j;
   __nv_bfloat16* yp = y + static_cast<long long>(i1) * ys2 + j;
-  for (int i0 = r0; i0 < r1; ++i0) {
-    const __nv_bfloat16 x1 = xp[i0 * xs1];
-    const __nv_bfloat16 x2 = xp[i0 * xs1 + half];
+  auto rotate_store = [&](__nv_bfloat16 x1, __nv_bfloat16 x2, int i0) {
     yp[i0 * ys1] = bsub(bmul(x1, c), bmul(x2, s));
     yp[i0 * ys1 + half] = badd(bmul(x2, c), bmul(x1, s));
+  };
+  // Rows at a time: their loads are issued before the first result is stored (a row's loads precede its own stores, and
+  // rows do not overlap).
+  constexpr int kRowsInFlight = 4;
+  int i0 = r0;
+  for (; i0 + kRowsInFlight <= r1; i0 += kRowsInFlight) {
+    __nv_bfloat16 x1[kRowsInFlight], x2[kRowsInFlight];
+#pragma unroll
+    for (int u = 0; u < kRowsInFlight; ++u) {
+      x1[u] = xp[(i0 + u) * xs1];
+      x2[u] = xp[(i0 + u) * xs1 + half];
+    }
+#pragma unroll
+    for (int u = 0; u < kRowsInFlight; ++u) rotate_store(x1[u], x2[u], i0 + u);
   }
+  for (; i0 < r1; ++i0) rotate_store(xp[i0 * xs1], xp[i0 * xs1 + half], i0);
 }
 
 constexpr int kRopeThreads = 256;
@@ -84,7 +100,7 @@ constexpr int kRopeMaxUnits = 128;  // units (position, eight adjacent pair indi
 // each once into shared memory, all threads sharing that work, and every row reads them from there. So a small d1 (the
 // query of a decode step: one position, four units) still runs with every thread busy on a row of its own, and a large
 // d1 can be cut into many short CTAs without paying for the trigonometry again in each thread.
-__global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* y,
+__global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8(const __nv_bfloat16* x, __nv_bfloat16* y,
                                                                  int pos, int d0, int d1, int d2, long long xs1,
                                                                  long long xs2, long long ys1, long long ys2, int units,
                                                                  int rows_per_block) {
@@ -143,10 +159,11 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8(const __nv_bflo
     *reinterpret_cast<uint4*>(yp + i0 * ys1) = o1;
     *reinterpret_cast<uint4*>(yp + i0 * ys1 + half) = o2;
   };
-  // Four rows at a time: their eight 16-byte loads are issued before the first result is stored, so a thread keeps
-  // 128 bytes in flight instead of 32 (in place is still fine: a row's loads precede its own stores, and rows do
-  // not overlap).
-  constexpr int kRowsInFlight = 4;
+  // Two rows at a time: their four 16-byte loads are issued before the first result is stored, so a thread keeps
+  // 64 bytes in flight instead of 32 (in place is still fine: a row's loads precede its own stores, and rows do
+  // not overlap). With four, most threads have no full set: 32 rows x 2049 positions 5.9 us against 4.9, 128 x 1024 8.8
+  // against 7.6.
+  constexpr int kRowsInFlight = 2;
   int i0 = r0 + tid / units;
   for (; i0 + (kRowsInFlight - 1) * step < r1; i0 += kRowsInFlight * step) {
     uint4 a[kRowsInFlight], b[kRowsInFlight];
@@ -166,9 +183,9 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8(const __nv_bflo
 }
 
 // The same for many units (the keys of a whole cache) or a single row: one unit per thread, its angles in registers, the
-// rows one after the other, so that the CTAs running together sweep few rows from end to end, which HBM likes best. The
-// keys of 128 rows x 6145 positions: 38.0 us; 44.2 in the kernel above with 256 units, 41 to 45 with 32 to 128.
-__global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8_wide(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* y, int pos,
+// rows one after the other. For many rows of a whole cache either kernel will do (128 rows x 6145 positions 38.6 us here, 38.2
+// above with 32 units), for few rows this one is faster (8 x 6145 4.3 against 5.4, 4 x 8192 3.65 against 3.8).
+__global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8_wide(const __nv_bfloat16* x, __nv_bfloat16* y, int pos,
                                                         int d0, int d1, int d2, long long xs1, long long xs2,
                                                         long long ys1, long long ys2, int rows_per_block) {
   const int half = d2 >> 1;
@@ -199,7 +216,8 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kernel_vec8_wide(const __nv
   const int r1 = min(d0, r0 + rows_per_block);
   const __nv_bfloat16* xp = x + static_cast<long long>(i1) * xs2 + j0;
   __nv_bfloat16* yp = y + static_cast<long long>(i1) * ys2 + j0;
-  constexpr int kRowsInFlight = 4;  // as above
+  // Two rows in flight: the keys of 128 rows x 6145 positions 38.4 us; one 44.3, three 41.2, four 40.3.
+  constexpr int kRowsInFlight = 2;
   // (packed arithmetic as above)
   __nv_bfloat162 c2[4], s2[4];
 #pragma unroll
@@ -476,8 +494,8 @@ int b200_mla_rope(const void* x, void* y, int pos, int d0, int d1, int d2, long 
                     (reinterpret_cast<uintptr_t>(x) % 16) == 0 && (reinterpret_cast<uintptr_t>(y) % 16) == 0;
   const long long pairs = static_cast<long long>(d1) * (vec8 ? half / 8 : half);
   // Units per CTA of the 16-byte kernels. Many units: one per thread (rope_kernel_vec8_wide). Fewer: 32, so that there
-  // are CTAs for every SM (2049 positions x 32 rows: 5.2 against 6.1 us); no more than there are, and no fewer than leave
-  // every row slot a row, up to one per thread again.
+  // are CTAs for every SM (2049 positions x 128 rows 13.5 against 15.7 us, x 32 4.95 against 5.3, x 8 2.4 against 3.9); no
+  // more than there are, and no fewer than leave every row slot a row, up to one per thread again.
   long long units = kRopeThreads;
   if (vec8 && pairs < kRopeWidePairs) {
     units = 1;

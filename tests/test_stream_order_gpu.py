@@ -104,3 +104,65 @@ def test_different_problems_back_to_back(seed):
     check_device_status()
     for g, w in zip(got, want):
         assert torch.equal(g, w)
+
+
+def adjacent(step, sync):
+    """Calls of this package one directly behind the other; each reads, some in place, what the one before wrote."""
+    m, n = 300, 512
+    a, b, a_s, b_s, c = pkg.make_inputs(m, n, 1024, seed=step, device="cuda")
+    c_aligned, c_odd = c, torch.zeros(m, n + 1, dtype=torch.bfloat16, device="cuda")[:, :n]
+    y = torch.zeros(m, n, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+
+    def calls():
+        yield lambda: pkg.custom_kernel((a, b, a_s, b_s, c_aligned))
+        yield lambda: pkg.mla_decode(c_aligned, c_aligned, step, 0, 0, m, 1, n, n, n, n, n)  # GEMM -> RoPE in place
+        yield lambda: pkg.mla_decode(c_aligned, y, step + 1, 0, 0, m, 1, n, n, n, n, n)      # RoPE -> RoPE out of place
+        yield lambda: pkg.div_softmax(y, 1, m, n, 128, 64)                                   # RoPE -> softmax
+        yield lambda: pkg.div_softmax(y, 1, 1, m * n, 1, 0)                                  # softmax -> softmax, other rows
+        yield lambda: pkg.custom_kernel((a, b, a_s, b_s, c_odd))
+        yield lambda: pkg.mla_decode(c_odd, c_odd, step, 0, 0, m, 1, n, n + 1, n + 1, n + 1, n + 1)  # the same, rows not aligned
+        yield lambda: pkg.custom_kernel((a, b, a_s, b_s, c_aligned))
+        yield lambda: pkg.div_softmax(c_aligned, 1, m, n, 1 << 16, 0)                        # GEMM -> softmax in place
+        yield lambda: pkg.mla_decode(c_aligned, c_aligned, step, 0, 0, 1, m, n, m * n, n, m * n, n)  # softmax -> RoPE, m positions
+
+    for call in calls():
+        call()
+        if sync:
+            torch.cuda.synchronize()
+    return [c_aligned, c_odd, y]
+
+
+@pytest.mark.parametrize("how", ["stream", "graph"])
+def test_directly_adjacent_calls(how):
+    for step in range(1, 9):
+        want = adjacent(step, sync=True)
+        got = adjacent(step, sync=False)
+        if how == "graph":
+            # the same calls once more, captured, on inputs of their own
+            m, n = 300, 512
+            a, b, a_s, b_s, c = pkg.make_inputs(m, n, 1024, seed=step, device="cuda")
+            s = torch.cuda.Stream()
+            torch.cuda.synchronize()
+            with torch.cuda.stream(s):
+                pkg.custom_kernel((a, b, a_s, b_s, c))  # (the stream's scratch exists before the capture)
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                for _ in range(4):
+                    pkg.custom_kernel((a, b, a_s, b_s, c))
+                    pkg.mla_decode(c, c, step, 0, 0, m, 1, n, n, n, n, n)
+                    pkg.div_softmax(c, 1, m, n, 1 << 16, 0)
+            g.replay()
+            torch.cuda.synchronize()
+            w = torch.zeros_like(c)
+            pkg.custom_kernel((a, b, a_s, b_s, w))
+            torch.cuda.synchronize()
+            pkg.mla_decode(w, w, step, 0, 0, m, 1, n, n, n, n, n)
+            torch.cuda.synchronize()
+            pkg.div_softmax(w, 1, m, n, 1 << 16, 0)
+            want, got = want + [w], got + [c]
+        torch.cuda.synchronize()
+        check_device_status()
+        for g_, w_ in zip(got, want):
+            assert torch.equal(g_.contiguous().view(torch.int16), w_.contiguous().view(torch.int16))
