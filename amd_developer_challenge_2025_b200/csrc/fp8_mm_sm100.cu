@@ -618,7 +618,9 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
   if (MODE == kGrouped) {
     while (true) {
       if (p.m_valid != nullptr) {
-        it.m_limit = max(0, min(p.M, __ldg(p.m_valid + cur.group)));
+        // (an ordinary load: the kernel before this one may have written the counts while this one's prologue ran, and
+        // read-only loads are not ordered after the wait for it)
+        it.m_limit = max(0, min(p.M, p.m_valid[cur.group]));
         tiles_m = (it.m_limit + tile_m - 1) / tile_m;
       }
       const int tiles = tiles_m * p.tiles_n;

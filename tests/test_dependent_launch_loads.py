@@ -9,7 +9,7 @@ import pytest
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "amd_developer_challenge_2025_b200", "csrc")
 
 
-@pytest.mark.parametrize("name", ["mla_consumers_sm100.cu"])
+@pytest.mark.parametrize("name", ["fp8_mm_sm100.cu", "mla_consumers_sm100.cu"])
 def test_no_read_only_loads(name):
     with open(os.path.join(CSRC, name)) as f:
         code = re.sub(r"//[^\n]*", "", f.read())

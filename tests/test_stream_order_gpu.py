@@ -166,3 +166,28 @@ def test_directly_adjacent_calls(how):
         check_device_status()
         for g_, w_ in zip(got, want):
             assert torch.equal(g_.contiguous().view(torch.int16), w_.contiguous().view(torch.int16))
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_row_counts_written_by_the_kernel_before(seed):
+    """Each grouped call's row counts are written by a call of this package directly before it: RoPE at position 0 leaves
+    every value as it is, so it copies the counts, seen as bf16 words, into the tensor that the grouped call is given."""
+    rng = random.Random(seed)
+    g, m, n, k = 8, 300, 320, 256
+    parts = [pkg.make_inputs(m, n, k, seed=i, device="cuda") for i in range(g)]
+    a, b, a_s, b_s = (torch.stack([p[j] for p in parts]) for j in range(4))
+    full = torch.zeros(g, m, n, dtype=torch.bfloat16, device="cuda")
+    pkg.fp8_mm_grouped(a, b, a_s, b_s, full)
+    rows = [[rng.randint(0, m) for _ in range(g)] for _ in range(12)]
+    counts = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    m_valid = torch.zeros(g, dtype=torch.int32, device="cuda")
+    outs = [torch.full_like(full, 7.0) for _ in rows]
+    w = 2 * g  # the counts as 16-bit words
+    torch.cuda.synchronize()
+    for i, c in enumerate(outs):
+        pkg.mla_decode(counts[i].view(torch.bfloat16), m_valid.view(torch.bfloat16), 0, 0, 0, 1, 1, w, w, w, w, w)
+        pkg.fp8_mm_grouped(a, b, a_s, b_s, c, m_valid=m_valid)
+    check_device_status()
+    for c, rs in zip(outs, rows):
+        for j, r in enumerate(rs):
+            assert torch.equal(c[j, :r], full[j, :r]) and bool((c[j, r:] == 7.0).all())
