@@ -13,7 +13,8 @@ ROOT = os.path.dirname(HERE)
 INCLUDE = os.path.join(ROOT, "include")
 SRC = os.path.join(HERE, "csrc", "fp8_mm_sm100.cu")
 SOURCES = [SRC, os.path.join(HERE, "csrc", "mla_consumers_sm100.cu")]
-HEADERS = [os.path.join(INCLUDE, "b200_fp8_mm.h"), os.path.join(INCLUDE, "b200_mla_consumers.h")]
+HEADERS = [os.path.join(INCLUDE, "b200_fp8_mm.h"), os.path.join(INCLUDE, "b200_mla_consumers.h"),
+           os.path.join(HERE, "csrc", "issuer_walk.h")]
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libb200fp8mm.so")
 HOST_SRC = os.path.join(HERE, "csrc", "host_calls.cpp")  # the entry points' per-call host work (a CPython module)

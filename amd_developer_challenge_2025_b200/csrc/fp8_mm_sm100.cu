@@ -18,8 +18,8 @@
 //               collects the promotion warps' release of the TMEM buffer that K block will
 //               overwrite (K block j uses stage j mod stages and buffer j mod buffers; a warp that
 //               has drained the buffer of K block j arrives on the barrier of K block j + buffers)
-//   warp 2      allocates / frees TMEM; its first lane is a second MMA issuer (the two issuers take
-//               alternate K blocks)
+//   warp 2      allocates / frees TMEM; its first lane is a second MMA issuer (the two issuers share
+//               the K blocks by ring stage, see issuer_walk.h)
 //   warp 3      scale loader: cp.async of the a_scale / b_scale values of FOUR K blocks at a time
 //               into a small shared-memory ring, up to 16 K blocks ahead
 //   warps 4-11  promotion + store: tcgen05.ld the partial, fma into register accumulators with
@@ -54,6 +54,7 @@
 #include <unordered_map>
 
 #include "b200_fp8_mm.h"
+#include "issuer_walk.h"
 
 namespace {
 
@@ -831,7 +832,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       __syncwarp();
     } else if (warp == 1 || warp == 2) {
       // ---------------- MMA issuers (the leader CTA of a pair issues for both) ----------------
-      // Up to two threads, one in each warp, take alternate K blocks. A K block's MMAs go to a TMEM
+      // Up to two threads, one in each warp, share the K blocks by ring stage. A K block's MMAs go to a TMEM
       // buffer of their own, so the two streams need no ordering between them; one thread alone spends
       // about 700 clocks per K block on its barrier wait and on issuing (an MMA costs the issuing
       // thread roughly 100 clocks), more than the tensor pipe needs for a narrow tile's block.
@@ -844,26 +845,24 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         const int me = warp - 1;
         const int total_work = work_total(), work_step = work_stride();
         const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_base_slot);
-        // Each issuer visits only its own K blocks (every issuers-th one of the CTA's whole sequence, across
-        // tile boundaries) and keeps its ring position with add-and-wrap only: no division and no work for
-        // the other issuer's blocks on this thread, whose scalar instructions are on the critical path.
-        const int step = p.issuers;
-        int my_stage = me % stages, my_buf = me % nbufs;
-        uint32_t my_phase = (me / stages) & 1u;
-        int first = me;  // offset of this issuer's next K block from the start of the next tile
+        // Each issuer visits only its own K blocks (see IssuerWalk, which runs on across tile boundaries) and keeps
+        // its ring position with add-and-wrap only: no division and no work for the other issuer's blocks on this
+        // thread, whose scalar instructions are on the critical path.
+        IssuerWalk at;
+        at.begin(me, stages, nbufs);
         bool ok = true;
         GroupCursor cursor{0, 0};
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
           const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
           if (MODE == kGrouped && it.done) break;
-          int kb = it.kb_begin + first;
-          for (; kb < it.kb_end; kb += step) {
-            const uint32_t sa = smem_u32(ring + my_stage * Cfg::kStageBytes);
+          const int blocks = it.kb_end - it.kb_begin;
+          while (at.block < blocks) {
+            const uint32_t sa = smem_u32(ring + at.stage * Cfg::kStageBytes);
             const uint32_t a_lo = smem_desc_addr(sa) | a_lo_bits;
             const uint32_t b_lo = smem_desc_addr(sa + Cfg::kStageBytesA) | b_lo_bits;
-            const uint32_t d_addr = tmem_base + static_cast<uint32_t>(my_buf * BN);
+            const uint32_t d_addr = tmem_base + static_cast<uint32_t>(at.buffer * BN);
             // operands landed AND the TMEM buffer of this K block drained (see the promotion warps)
-            if (!mbar_wait(smem_u32(&full_bar[my_stage]), my_phase, ctx, 0x300 | my_stage)) {
+            if (!mbar_wait(smem_u32(&full_bar[at.stage]), at.phase, ctx, 0x300 | at.stage)) {
               ok = false;
               break;
             }
@@ -875,16 +874,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
               umma_f8<PAIR>(d_addr, a_lo + a_kstep * k, b_lo + b_kstep * k, a_hi, b_hi, idesc, k > 0 ? 1u : 0u);
             }
 #endif
-            umma_commit<PAIR>(smem_u32(&done_bar[my_stage]));
-            my_stage += step;
-            if (my_stage >= stages) {
-              my_stage -= stages;
-              my_phase ^= 1u;
-            }
-            my_buf += step;
-            while (my_buf >= nbufs) my_buf -= nbufs;
+            umma_commit<PAIR>(smem_u32(&done_bar[at.stage]));
+            at.next(me, p.issuers, stages, nbufs);
           }
-          first = kb - it.kb_end;
+          at.block -= blocks;
         }
       }
       __syncwarp();
