@@ -46,6 +46,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
@@ -88,8 +89,8 @@ struct KernelParams {
   int full_tiles;  // tiles [0, full_tiles) run unsplit; the rest are split split_k ways along K
   int raster_group;
   // Reciprocals for decode_work's divisions (see div_small): 1 / (raster_group * tiles_n), 1 / raster_group,
-  // 1 / (rows of the last, shorter raster group), 1 / split_k.
-  float rcp_per_group, rcp_raster, rcp_raster_last, rcp_split;
+  // 1 / (rows of the last, shorter raster group), 1 / split_k, 1 / (tiles_m * tiles_n), 1 / tiles_n.
+  float rcp_per_group, rcp_raster, rcp_raster_last, rcp_split, rcp_per_problem, rcp_tiles_n;
   int b_scale_rows;
   int vec_store;  // 1 when c, ldc and N allow 16-byte stores
   int stages;
@@ -109,6 +110,10 @@ struct KernelParams {
   // Grouped launches (groups > 0): M, tiles_m, a_scale/b_scale/c strides are per group.
   int groups;
   const int* m_valid;        // device int[groups]: rows of each group that exist (null: all M)
+  int group_marks;           // with m_valid: offset of the table of marks (see kGroupMarks) from the barriers, bytes
+  int groups_per_mark, num_marks;  // groups of an entry; entries in use
+  int item_list, item_slots;       // offset of a grouped launch's list of decoded items, and how many it takes
+  int items_each, items_more;      // items of a CTA (or pair) of a grouped launch; the first `items_more` have one more
   long long sa_g, sb_g, c_g; // group strides of a_scale, b_scale (floats) and c (elements)
   unsigned long long wait_limit_ns;  // every mbarrier wait gives up after this long
   // Self-test of the give-up path (b200_fp8_mm_selftest_wait_expiry): the producer of the plain 64-wide
@@ -564,11 +569,25 @@ struct WorkItem {
   bool done;    // past the end of the work list (grouped launches; the others know their extent beforehand)
 };
 
-// Where a role stands in a grouped launch's work list: the tiles of groups before `group` take indices [0, base).
-// A role's work indices only grow, so it moves through the groups once per launch.
-struct GroupCursor {
-  int group, base;
-};
+// A grouped launch with row counts keeps a table in shared memory, one mark per group or, where there are more groups than
+// marks, per run of `groups_per_mark` groups: (tile rows before it) << 8 | (rows of the group's last tile - 1). A launch has
+// at most 2^20 tile rows. Marks that are not in use hold INT_MAX. Beside them, in the header: every sixteenth mark once more
+// and the number of tile rows in all.
+constexpr int kGroupMarks = 256;
+constexpr int kGroupMarkBytes = kGroupMarks * 4;
+constexpr int kGroupTopOffset = kBarrierBytes + kScaleSlots * kScaleSlotFloats * 4;
+static_assert(kGroupTopOffset % 16 == 0 && kGroupTopOffset + (kGroupMarks / 16 + 1) * 4 <= kHeaderBytes, "no room in the header");
+
+// A grouped launch decodes a CTA's first work items once, in parallel, into a shared-memory list {group, m0, n0, m_limit};
+// each role then reads its next item there. The list lies behind the marks where there is room for it (at 192 columns there may
+// be none, then a few items lie in the header). Items beyond it are decoded by each role for itself. When every role walked the
+// list of groups by itself, one global load a group, 256 groups x 16 x 256 x 256 took 28.9 us (now 11.1, without counts 18.4 and
+// 10.1), 256 x 128 x 512 x 512 39.7 (23.3), 1024 x 16 x 256 x 128 101 (22.2); 8 x 1024 x 2048 x 7168 with uneven loads 100.4
+// (100.9).
+constexpr int kMaxItemSlots = 384;  // one per thread
+constexpr int kHeaderItemSlots = 8;
+constexpr int kHeaderItemOffset = kGroupTopOffset + 80;
+static_assert(kHeaderItemOffset % 16 == 0 && kHeaderItemOffset + kHeaderItemSlots * 16 <= kHeaderBytes, "no room in the header");
 
 // n / d for 0 <= n < 2^22 and d >= 1, with rcp = 1.0f / d: the float quotient is off by at most one, which the
 // remainder corrects. Every role decodes one work item per tile; the hardware has no integer divide, and the
@@ -586,15 +605,67 @@ __device__ __forceinline__ int div_small(int n, int d, float rcp) {
 }
 constexpr int kDivSmallLimit = 1 << 22;
 
+// Rows of group g that exist. (An ordinary load: the kernel before this one may have written the counts while this one's
+// prologue ran, and read-only loads are not ordered after the wait for it.)
+__device__ __forceinline__ int group_rows(const KernelParams& p, int g) { return max(0, min(p.M, p.m_valid[g])); }
+
+// The group that tile row r of a grouped launch with row counts lies in, the tile rows before that group and the group's
+// rows; false when r is past the end. The run of groups is the last one with no more than r tile rows before it; the marks
+// never fall, so their count is its place: first every sixteenth mark is counted, then the sixteen from there on. Beyond 256
+// groups the group is then looked for in its run.
+__device__ __forceinline__ bool find_group(const KernelParams& p, const int* marks, const int* top, int r, int tile_m,
+                                           int* group, int* before, int* rows) {
+  const int total = top[kGroupMarks / 16];
+  if (r >= total) return false;
+  const int key = (r << 8) | 255;
+  auto upto = [&](const int* at) {
+    int count = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int4 v = reinterpret_cast<const int4*>(at)[i];
+      count += (v.x <= key) + (v.y <= key) + (v.z <= key) + (v.w <= key);
+    }
+    return count;
+  };
+  const int first = p.num_marks > 16 ? 16 * (upto(top) - 1) : 0;
+  const int e = first + upto(marks + first) - 1;
+  const int mark = marks[e];
+  int base = mark >> 8;
+  if (p.groups_per_mark == 1) {
+    const int next = e + 1 < p.num_marks ? marks[e + 1] >> 8 : total;
+    *group = e;
+    *before = base;
+    *rows = (next - base - 1) * tile_m + (mark & 255) + 1;
+    return true;
+  }
+  for (int g = e * p.groups_per_mark; g < p.groups; g += 4) {  // (ends sooner: the run holds tile row r)
+    int mine[4];  // four loads in flight
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mine[i] = g + i < p.groups ? group_rows(p, g + i) : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int tiles = (mine[i] + tile_m - 1) / tile_m;
+      if (r - base < tiles) {
+        *group = g + i;
+        *before = base;
+        *rows = mine[i];
+        return true;
+      }
+      base += tiles;
+    }
+  }
+  return false;
+}
+
 // Work item w -> tile and K range. Tiles are walked in groups of raster_group tile rows, column
 // by column inside a group, so that the CTAs running at one time share A and B tiles in L2.
 //
-// A grouped launch lists only tiles that hold rows: group after group, ceil(valid rows / tile rows) tile rows each, so
-// the row counts (device memory, unknown to the host) decide how many items there are and every CTA gets an equal
-// share of them. With the empty tiles listed and skipped, the CTAs' shares of real ones differed by up to one in
+// A grouped launch with row counts lists only tiles that hold rows: group after group, ceil(valid rows / tile rows) tile
+// rows each, so the row counts (device memory, unknown to the host) decide how many items there are and every CTA gets an
+// equal share of them. With the empty tiles listed and skipped, the CTAs' shares of real ones differed by up to one in
 // three (8 x 1024 x 2048 x 7168 with loads of 1/8 .. 8/8: 160 real tiles of 256 on 74 pairs, four for some and one for others).
 template <int MODE>
-__device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, int tile_m, int block_n, GroupCursor& cur) {
+__device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, int tile_m, int block_n, const int* marks, const int* top) {
   WorkItem it;
   int t;
   it.done = false;
@@ -616,24 +687,20 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
   it.group = 0;
   it.m_limit = p.M;
   int tiles_m = p.tiles_m;
-  if (MODE == kGrouped) {
-    while (true) {
-      if (p.m_valid != nullptr) {
-        // (an ordinary load: the kernel before this one may have written the counts while this one's prologue ran, and
-        // read-only loads are not ordered after the wait for it)
-        it.m_limit = max(0, min(p.M, p.m_valid[cur.group]));
-        tiles_m = (it.m_limit + tile_m - 1) / tile_m;
-      }
-      const int tiles = tiles_m * p.tiles_n;
-      if (w - cur.base < tiles) break;
-      cur.base += tiles;
-      if (++cur.group == p.groups) {
-        it.done = true;
-        return it;
-      }
+  if (MODE == kGrouped && p.m_valid == nullptr) {
+    const int per_problem = p.tiles_m * p.tiles_n;
+    it.group = small ? div_small(t, per_problem, p.rcp_per_problem) : t / per_problem;
+    t -= it.group * per_problem;
+    small = t < kDivSmallLimit;
+  } else if (MODE == kGrouped) {
+    const int r = small ? div_small(t, p.tiles_n, p.rcp_tiles_n) : t / p.tiles_n;
+    int base;
+    if (!find_group(p, marks, top, r, tile_m, &it.group, &base, &it.m_limit)) {
+      it.done = true;
+      return it;
     }
-    it.group = cur.group;
-    t = w - cur.base;
+    tiles_m = (it.m_limit + tile_m - 1) / tile_m;
+    t -= base * p.tiles_n;
     small = t < kDivSmallLimit;
   }
   const int per_group = p.raster_group * p.tiles_n;
@@ -643,7 +710,10 @@ __device__ __forceinline__ WorkItem decode_work(const KernelParams& p, int w, in
   const int gsize = whole ? p.raster_group : tiles_m - first_m;
   const int within = t - group * per_group;
   float rcp_gsize = whole ? p.rcp_raster : p.rcp_raster_last;
-  if (MODE == kGrouped && !whole) rcp_gsize = __frcp_rn(static_cast<float>(gsize));  // a group's own last rows
+  if (MODE == kGrouped && !whole && tiles_m != p.tiles_m) {  // a group's own last rows
+    // (off by an ulp at most, which leaves div_small's quotient off by at most one)
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rcp_gsize) : "f"(static_cast<float>(gsize)));
+  }
   const int tn = small ? div_small(within, gsize, rcp_gsize) : within / gsize;
   const int tm = first_m + (within - tn * gsize);
   it.m0 = tm * tile_m;
@@ -693,6 +763,9 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(scale_empty_bar + kScaleSlots);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 1);
   volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_base_slot + 2);
+  int* const marks = reinterpret_cast<int*>(smem + (MODE == kGrouped ? p.group_marks : 0));
+  int* const top = reinterpret_cast<int*>(smem + kGroupTopOffset);
+  int4* const item_list = reinterpret_cast<int4*>(smem + (MODE == kGrouped ? p.item_list : 0));
   // staging for the TMA store of c: [warpgroup][buffer][128 rows x 64 B], behind the ring (1024-byte aligned:
   // the header and every stage are multiples of 1024 bytes)
   uint8_t* staging = ring + stages * Cfg::kStageBytes;
@@ -702,6 +775,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   const AbortCtx ctx{abort_flag, p.status, p.wait_limit_ns};
   const uint32_t cta_rank = PAIR ? cluster_ctarank() : 0u;
 
+  if (MODE == kGrouped && p.m_valid != nullptr)
+    for (int e = static_cast<int>(threadIdx.x); e < kGroupMarks; e += Cfg::kThreads) marks[e] = 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
       // one arrive.expect_tx per producing CTA + one release per promotion warp (of both CTAs)
@@ -744,18 +819,85 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
   // take the SMs that this kernel's CTAs leave, and wait there.
   pdl_wait();
   pdl_launch_dependents();
-  // The TMEM base address is read again inside each role instead of being carried across the register
-  // re-allocation below: a value that is live in every role at once gets one register for all of them, which
-  // the promotion warps' accumulators then push out to local memory for everybody.
-
-  // The extent of the work list (kept out of registers across the role split for the same reason).
+  if (MODE == kGrouped && p.m_valid != nullptr) {
+    // The table: tile rows of each run of groups, then their exclusive sums.
+    for (int g = static_cast<int>(threadIdx.x); g < p.groups; g += Cfg::kThreads) {
+      const int rows = group_rows(p, g);
+      const int tile_rows = (rows + Cfg::kTileM - 1) / Cfg::kTileM;
+      if (p.groups_per_mark == 1) {
+        marks[g] = (tile_rows << 8) | ((rows - 1) & (Cfg::kTileM - 1));
+      } else {
+        atomicAdd(&marks[g / p.groups_per_mark], tile_rows << 8);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      constexpr int kEach = kGroupMarks / 32;
+      int mine[kEach], sum = 0;
+#pragma unroll
+      for (int i = 0; i < kEach; ++i) {
+        mine[i] = marks[lane * kEach + i];
+        sum += mine[i] >> 8;
+      }
+      int upto = sum;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += v;
+      }
+      int before = upto - sum;
+#pragma unroll
+      for (int i = 0; i < kEach; ++i) {
+        const int e = lane * kEach + i;
+        const int v = e < p.num_marks ? (before << 8) | (mine[i] & 255) : INT_MAX;
+        before += mine[i] >> 8;
+        marks[e] = v;
+        if (e % 16 == 0) top[e / 16] = v;
+      }
+      if (lane == 31) top[kGroupMarks / 16] = upto;
+    }
+    __syncthreads();
+  }
+  // This CTA's share of the work list (kept out of registers across the role split for the reason below): items work_begin(),
+  // + work_stride(), ... < work_total(). A grouped launch counts the CTA's own items 0, 1, ... instead, of which the last may
+  // be past the end of the list (WorkItem::done).
+  auto first_item = [&]() { return PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x); };
+  auto item_stride = [&]() { return PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x); };
   auto work_total = [&]() {
-    if (MODE == kGrouped) return p.full_tiles;  // the most there can be; see WorkItem::done
+    if (MODE == kGrouped) return p.items_each + (first_item() < p.items_more ? 1 : 0);
     const int all_tiles = p.tiles_m * p.tiles_n;
     return p.full_tiles + (all_tiles - p.full_tiles) * p.split_k;
   };
-  auto work_begin = [&]() { return PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x); };
-  auto work_stride = [&]() { return PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x); };
+  auto work_begin = [&]() { return MODE == kGrouped ? 0 : first_item(); };
+  auto work_stride = [&]() { return MODE == kGrouped ? 1 : item_stride(); };
+  auto work_item = [&](int w) {
+    if (MODE != kGrouped) return decode_work<MODE>(p, w, Cfg::kTileM, BN, marks, top);
+    if (w >= p.item_slots) return decode_work<MODE>(p, first_item() + w * item_stride(), Cfg::kTileM, BN, marks, top);
+    WorkItem it;
+    const int4 v = item_list[w];
+    it.group = v.x;
+    it.m0 = v.y;
+    it.n0 = v.z;
+    it.m_limit = v.w;
+    it.done = v.x < 0;
+    it.tile = 0;
+    it.split = 0;
+    it.nsplit = 1;
+    it.kb_begin = 0;
+    it.kb_end = p.kblocks;
+    return it;
+  };
+  if (MODE == kGrouped) {
+    const int w = static_cast<int>(threadIdx.x);
+    if (w < p.item_slots && w < work_total()) {
+      const WorkItem it = decode_work<MODE>(p, first_item() + w * item_stride(), Cfg::kTileM, BN, marks, top);
+      item_list[w] = it.done ? make_int4(-1, 0, 0, 0) : make_int4(it.group, it.m0, it.n0, it.m_limit);
+    }
+    __syncthreads();
+  }
+  // The TMEM base address is read again inside each role instead of being carried across the register
+  // re-allocation below: a value that is live in every role at once gets one register for all of them, which
+  // the promotion warps' accumulators then push out to local memory for everybody.
 
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsLight));
@@ -766,9 +908,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        GroupCursor cursor{0, 0};
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
-          const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+          const WorkItem it = work_item(w);
           if (MODE == kGrouped && it.done) break;
           const int a_row = it.m0 + static_cast<int>(cta_rank) * kBlockM;
           const int b_row = it.n0 + static_cast<int>(cta_rank) * (PAIR ? Cfg::kRowsB : 0);
@@ -851,9 +992,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         IssuerWalk at;
         at.begin(me, stages, nbufs);
         bool ok = true;
-        GroupCursor cursor{0, 0};
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
-          const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+          const WorkItem it = work_item(w);
           if (MODE == kGrouped && it.done) break;
           const int blocks = it.kb_end - it.kb_begin;
           while (at.block < blocks) {
@@ -889,9 +1029,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       int slot = 0;
       uint32_t sphase = 0;
       bool ok = true;
-      GroupCursor cursor{0, 0};
       for (int w = work_begin(); w < total_work && ok; w += work_step) {
-        const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+        const WorkItem it = work_item(w);
         if (MODE == kGrouped && it.done) break;
         const int row0 = it.m0 + static_cast<int>(cta_rank) * kBlockM;
         const float* a_base = p.a_scale + static_cast<long long>(it.group) * p.sa_g;
@@ -978,9 +1117,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     // warp then stops waiting, fetching and storing but still walks the remaining tiles and takes part in
     // every named barrier of their epilogues, so that warps which have not noticed yet are never left alone
     // at a barrier; they notice at their next wait.
-    GroupCursor cursor{0, 0};
     for (int w = work_begin(); w < total_work; w += work_step) {
-      const WorkItem it = decode_work<MODE>(p, w, Cfg::kTileM, BN, cursor);
+      const WorkItem it = work_item(w);
       if (MODE == kGrouped && it.done) break;
       const int row = it.m0 + static_cast<int>(cta_rank) * kBlockM + row_in_tile;
       // Index of this thread's first b_scale row inside a ring slot (at most 2 rows per 128 columns).
@@ -1351,8 +1489,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     cluster_sync_all();
     if (warp >= 4 && *abort_flag == 0) {
       const int ranges = p.split_k;
-      GroupCursor cursor{0, 0};
-      const WorkItem it = decode_work<MODE>(p, static_cast<int>(blockIdx.x), Cfg::kTileM, BN, cursor);
+      const WorkItem it = decode_work<MODE>(p, static_cast<int>(blockIdx.x), Cfg::kTileM, BN, marks, top);
       constexpr int kPieces = BN / 4;  // per row
       const int rows = min(kBlockM, p.M - it.m0);
       const uint32_t base = smem_u32(ring);
@@ -1849,6 +1986,8 @@ void set_decode_reciprocals(KernelParams& kp) {
   kp.rcp_raster = 1.0f / static_cast<float>(kp.raster_group);
   kp.rcp_raster_last = 1.0f / static_cast<float>(last > 0 ? last : kp.raster_group);
   kp.rcp_split = 1.0f / static_cast<float>(kp.split_k > 0 ? kp.split_k : 1);
+  kp.rcp_per_problem = 1.0f / static_cast<float>(kp.tiles_m * kp.tiles_n);
+  kp.rcp_tiles_n = 1.0f / static_cast<float>(kp.tiles_n);
 }
 
 // decode_work forms (split + 1) * kblocks in 32 bits; the selector itself never splits more than 16 ways.
@@ -2255,12 +2394,35 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.sa_g = sa_g;
   kp.sb_g = sb_g;
   kp.c_g = c_g;
+  // The list of decoded items and, with row counts, the marks lie behind everything the plan counts. Rings and staging come in
+  // multiples of 4 KiB, so a plan that fits leaves at least the marks' 1 KiB of the 227 KiB.
+  static_assert((kMaxSmem - 1024 - kHeaderBytes) % 4096 >= kGroupMarkBytes, "no room for the marks");
+  static_assert(kMaxItemSlots <= TileCfg<64, false>::kThreads, "one item per thread");
+  if (m_valid != nullptr) {
+    kp.group_marks = pl.smem_bytes - 1024;  // (less the alignment slack)
+    pl.smem_bytes += kGroupMarkBytes;
+    kp.groups_per_mark = ceil_div(groups, kGroupMarks);
+    kp.num_marks = ceil_div(groups, kp.groups_per_mark);
+  }
   pl.tiles = kp.full_tiles;
   pl.full_tiles = kp.full_tiles;
   {
     const int units = pl.cta_pair ? sm_count / 2 : sm_count;
     const int used = kp.full_tiles < units ? kp.full_tiles : units;
     pl.grid = pl.cta_pair ? 2 * used : used;
+    kp.items_each = kp.full_tiles / used;
+    kp.items_more = kp.full_tiles % used;
+    kp.item_slots = kp.items_each + (kp.items_more > 0 ? 1 : 0);
+  }
+  if (kp.item_slots > kMaxItemSlots) kp.item_slots = kMaxItemSlots;
+  const int room = (kMaxSmem - pl.smem_bytes) / 16;
+  if (kp.item_slots > room && room < kHeaderItemSlots) {
+    kp.item_list = kHeaderItemOffset;
+    kp.item_slots = kHeaderItemSlots;
+  } else {
+    if (kp.item_slots > room) kp.item_slots = room;
+    kp.item_list = pl.smem_bytes - 1024;
+    pl.smem_bytes += kp.item_slots * 16;
   }
   return launch(fn, pl, pl.cta_pair ? 2 : 1, map_a, map_b, map_c, kp, stream);
 }
