@@ -2068,6 +2068,26 @@ int sm_count_for_sizing() {
   return n > 0 ? n : 148;
 }
 
+// A workspace that run() accepts for this problem with this forced plan (or none), whichever way it goes: the demand of the
+// plan before a cluster plan replaces it (choose_plan's workspace_need), the final plan's size as a split plan, and both
+// again for the single-CTA plan that MN-major operands may be given instead of a pair plan.
+size_t workspace_bytes_for(int M, int N, int K, int sm_count, const b200_fp8_mm_plan* forced) {
+  b200_fp8_mm_plan single;
+  memset(&single, 0, sizeof(single));
+  if (forced != nullptr) single = *forced;
+  size_t most = 0;
+  for (int pass = 0; pass < 2; ++pass) {
+    b200_fp8_mm_plan pl;
+    size_t need = 0;
+    choose_plan(M, N, K, sm_count, pass == 0 ? forced : &single, &pl, &need);
+    if (need > most) most = need;
+    if (plan_workspace_bytes(pl) > most) most = plan_workspace_bytes(pl);
+    if (forced != nullptr && forced->cta_pair > 0) break;  // a forced pair plan is run or refused, never replaced
+    single.cta_pair = -1;
+  }
+  return ((most + 255) / 256) * 256;
+}
+
 int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUtensorMap& map_a, const CUtensorMap& map_b,
            const CUtensorMap& map_c, const KernelParams& kp, void* stream);
 
@@ -2546,28 +2566,12 @@ size_t b200_fp8_mm_static_scratch_limit(void) { return kStaticScratchBytes; }
 
 size_t b200_fp8_mm_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0 || (K % kBlockK) != 0) return 0;
-  // Covers both the plan for K-major operands and the one for MN-major operands (no CTA pairs).
-  b200_fp8_mm_plan pl, single;
-  const int sms = sm_count_for_sizing();
-  size_t need = 0, need2 = 0;
-  choose_plan(M, N, K, sms, nullptr, &pl, &need);
-  memset(&single, 0, sizeof(single));
-  single.cta_pair = -1;
-  b200_fp8_mm_plan pl2;
-  choose_plan(M, N, K, sms, &single, &pl2, &need2);
-  if (need2 > need) need = need2;
-  // (a plan that runs as clusters needs none of this, but its size as a split plan is covered all the same)
-  if (plan_workspace_bytes(pl) > need) need = plan_workspace_bytes(pl);
-  if (plan_workspace_bytes(pl2) > need) need = plan_workspace_bytes(pl2);
-  return ((need + 255) / 256) * 256;
+  return workspace_bytes_for(M, N, K, sm_count_for_sizing(), nullptr);
 }
 
 size_t b200_fp8_mm_plan_workspace_bytes(int M, int N, int K, const b200_fp8_mm_plan* forced) {
   if (M <= 0 || N <= 0 || K <= 0 || (K % kBlockK) != 0) return 0;
-  b200_fp8_mm_plan pl;
-  choose_plan(M, N, K, sm_count_for_sizing(), forced, &pl);
-  const size_t need = plan_workspace_bytes(pl);
-  return ((need + 255) / 256) * 256;
+  return workspace_bytes_for(M, N, K, sm_count_for_sizing(), forced);
 }
 
 int b200_fp8_mm_describe(int M, int N, int K, int n_phase, int sm_count, b200_fp8_mm_plan* out) {
