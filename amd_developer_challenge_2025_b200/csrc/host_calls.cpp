@@ -141,6 +141,13 @@ bool ints(PyObject* const* args, int count, long long limit, long long* out) {
   return true;
 }
 
+// Whether the elements off + [0, span1] + [0, span2] + [0, row) lie inside the bf16 tensor's storage (spans of either sign).
+bool inside(const at::Tensor& t, long long off, long long span1, long long span2, long long row) {
+  const long long first = off + (span1 < 0 ? span1 : 0) + (span2 < 0 ? span2 : 0);
+  const long long last = off + (span1 > 0 ? span1 : 0) + (span2 > 0 ? span2 : 0) + row - 1;
+  return t.storage_offset() + first >= 0 && t.storage_offset() + last < static_cast<long long>(t.storage().nbytes() / 2);
+}
+
 // mla_decode(x, y, pos, xoff, yoff, d0, d1, d2, xs1, xs2, ys1, ys2)
 bool run_rope(PyObject* const* args) {
   const at::Tensor *x = plain_tensor(args[0]), *y = plain_tensor(args[1]);
@@ -157,11 +164,7 @@ bool run_rope(PyObject* const* args) {
   if (d0 <= 0 || d1 <= 0 || d2 <= 0 || d2 % 2 != 0 || d0 > (1 << 20) || d1 > (1 << 20) || d2 > (1 << 20) ||
       pos > 0x7fffffff || pos < -0x7fffffff || xoff < 0 || yoff < 0)
     return false;
-  const long long last_x = xoff + (d0 - 1) * xs1 + (d1 - 1) * xs2 + d2 - 1;
-  const long long last_y = yoff + (d0 - 1) * ys1 + (d1 - 1) * ys2 + d2 - 1;
-  if (last_x >= static_cast<long long>(x->storage().nbytes() / 2) - x->storage_offset() ||
-      last_y >= static_cast<long long>(y->storage().nbytes() / 2) - y->storage_offset())
-    return false;
+  if (!inside(*x, xoff, (d0 - 1) * xs1, (d1 - 1) * xs2, d2) || !inside(*y, yoff, (d0 - 1) * ys1, (d1 - 1) * ys2, d2)) return false;
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   return launched(g_rope, static_cast<char*>(x->data_ptr()) + 2 * xoff, static_cast<char*>(y->data_ptr()) + 2 * yoff,
                 static_cast<int>(pos), static_cast<int>(d0), static_cast<int>(d1), static_cast<int>(d2), xs1, xs2, ys1,

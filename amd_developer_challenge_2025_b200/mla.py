@@ -12,6 +12,16 @@ from . import _lib
 from .fp8_mm import Fp8MmError, _check, fp8_mm
 
 
+def _check_range(name, t, off, d0, d1, d2, s1, s2):
+    """Every element off + i0*s1 + i1*s2 + j (strides of either sign) lies inside t's storage."""
+    spans = ((d0 - 1) * s1, (d1 - 1) * s2)
+    first = off + sum(min(0, v) for v in spans)
+    last = off + sum(max(0, v) for v in spans) + d2 - 1
+    start = t.storage_offset()
+    _check(0 <= off and 0 <= start + first and start + last < t.untyped_storage().nbytes() // t.element_size(),
+           f"{name}: range outside the tensor")
+
+
 def mla_decode(x, y, pos: int, xoff: int, yoff: int, d0: int, d1: int, d2: int, xs1: int, xs2: int, ys1: int,
                ys2: int):
     """Rotary position embedding, the reference's `module.mla_decode`: reads the bf16 elements
@@ -23,11 +33,8 @@ def mla_decode(x, y, pos: int, xoff: int, yoff: int, d0: int, d1: int, d2: int, 
     _check(x.is_cuda and y.is_cuda and x.device == y.device, "x and y must be CUDA tensors on one device")
     _check(x.dtype == torch.bfloat16 and y.dtype == torch.bfloat16, "x and y must be bfloat16")
     _check(d0 > 0 and d1 > 0 and d2 > 0 and d2 % 2 == 0, "d0, d1, d2 must be positive and d2 even")
-    # the last element touched must lie inside each tensor's storage
-    last_x = xoff + (d0 - 1) * xs1 + (d1 - 1) * xs2 + d2 - 1
-    last_y = yoff + (d0 - 1) * ys1 + (d1 - 1) * ys2 + d2 - 1
-    _check(0 <= xoff and last_x < x.untyped_storage().nbytes() // 2 - x.storage_offset(), "x: range outside the tensor")
-    _check(0 <= yoff and last_y < y.untyped_storage().nbytes() // 2 - y.storage_offset(), "y: range outside the tensor")
+    _check_range("x", x, xoff, d0, d1, d2, xs1, xs2)
+    _check_range("y", y, yoff, d0, d1, d2, ys1, ys2)
     with torch.cuda.device(x.device):
         rc = _lib.load().b200_mla_rope(x.data_ptr() + 2 * xoff, y.data_ptr() + 2 * yoff, pos, d0, d1, d2, xs1, xs2, ys1,
                                        ys2, torch.cuda.current_stream(x.device).cuda_stream)

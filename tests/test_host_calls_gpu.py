@@ -110,3 +110,23 @@ def test_other_types_of_argument_are_left_to_python(stubs):
     assert not native.fp8_mm_grouped(g[0][:1], *g[1:], None, host._status)
     assert not native.fp8_mm_grouped(*p, None, host._status)
     assert len(stubs) == 4
+
+
+@pytest.mark.parametrize("xs1,xs2,xoff,ok", [(64, 64, 0, True), (-64, 64, 448, True), (-64, 64, 447, False), (-64, 64, 0, False),
+                                             (64, -64, 128, True), (64, -64, 127, False), (-64, -64, 576, True),
+                                             (-64, -64, 575, False), (64, -64, 129, False),
+                                             (-(1 << 40), 64, 0, False), (64, -(1 << 40), 448, False)])
+def test_rope_strides_of_either_sign(stubs, xs1, xs2, xoff, ok):
+    """8 x 3 rows of 64 in a tensor of 640 elements: rows before its start or past its end are refused, as x and as y."""
+    t, whole = torch.zeros(640, dtype=torch.bfloat16, device="cuda"), torch.zeros(8, 3, 64, dtype=torch.bfloat16, device="cuda")
+    native = _lib.host_calls()
+    assert native.mla_decode(t, whole, 0, xoff, 0, 8, 3, 64, xs1, xs2, 192, 64) == ok
+    assert native.mla_decode(whole, t, 0, 0, xoff, 8, 3, 64, 192, 64, xs1, xs2) == ok
+    assert len(stubs) == 2 * int(ok)
+    if not ok:
+        import amd_developer_challenge_2025_b200 as pkg
+        with pytest.raises(ValueError, match="x: range outside"):
+            pkg.mla_decode(t, whole, 0, xoff, 0, 8, 3, 64, xs1, xs2, 192, 64)
+        with pytest.raises(ValueError, match="y: range outside"):
+            pkg.mla_decode(whole, t, 0, 0, xoff, 8, 3, 64, 192, 64, xs1, xs2)
+        assert len(stubs) == 0
