@@ -135,8 +135,9 @@ bool run_grouped(PyObject* const* args) {
 bool ints(PyObject* const* args, int count, long long limit, long long* out) {
   for (int i = 0; i < count; ++i) {
     if (!PyLong_CheckExact(args[i])) return false;
-    out[i] = PyLong_AsLongLong(args[i]);
-    if (out[i] > limit || out[i] < -limit) return false;
+    int overflow = 0;
+    out[i] = PyLong_AsLongLongAndOverflow(args[i], &overflow);  // (beyond 64 bits the value itself would read as -1)
+    if (overflow != 0 || out[i] > limit || out[i] < -limit) return false;
   }
   return true;
 }

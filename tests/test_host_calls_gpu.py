@@ -130,3 +130,20 @@ def test_rope_strides_of_either_sign(stubs, xs1, xs2, xoff, ok):
         with pytest.raises(ValueError, match="y: range outside"):
             pkg.mla_decode(whole, t, 0, 0, xoff, 8, 3, 64, 192, 64, xs1, xs2)
         assert len(stubs) == 0
+
+
+@pytest.mark.parametrize("big", [1 << 62, 1 << 64, -(1 << 64), 1 << 100])
+def test_integers_beyond_64_bits_launch_nothing(stubs, big):
+    native = _lib.host_calls()
+    q = torch.zeros(8, 1, 64, dtype=torch.bfloat16, device="cuda")
+    ok = (q, q, 5, 64, 64, 7, 1, 64, 64, 64, 64, 64)
+    for i in range(2, 12):
+        assert not native.mla_decode(*ok[:i], big, *ok[i + 1:])
+    s = torch.zeros(2, 3, 5, dtype=torch.bfloat16, device="cuda")
+    for i in range(1, 6):
+        call = [s, 2, 3, 5, 128, 64]
+        call[i] = big
+        assert not native.div_softmax(*call)
+    p = parts()
+    assert not native.fp8_mm(*p, big, host._workspaces, host._status)
+    assert stubs == []
