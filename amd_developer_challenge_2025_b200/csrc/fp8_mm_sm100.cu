@@ -1951,10 +1951,10 @@ double choose_plan(int M, int N, int K, int sm_count, const b200_fp8_mm_plan* fo
   // 64-wide pairs halve what a CTA loads of b per K block but take longer to start and to finish: below about 20 K blocks
   // single CTAs are faster (1024 x 1024 x 1024 5.7 against 6.5 us, 300 x 2000 x 512 4.7 against 5.6, 129 x 4099 x 2304 10.7
   // against 11.5), from there on they are not (200 x 2000 x 2560 8.5 against 8.4, 900 x 256 x 6144 15.1 against 14.7).
-  if (f_pair < 0 && best.pair && best.bn == 64 && best.split == 1 && kblocks < 20) {
-    best.pair = 0;
-    best.full_tiles = ceil_div(M, kBlockM) * ceil_div(N, best.bn);
-  }
+  // (They stay ahead of the wider tiles that the pair was ahead of: 909 x 2325 x 1152 13.5 us, 192-wide pairs 16.8. From here on
+  // the cost is the single-CTA plan's own, so that it is what clusters have to beat: 945 x 541 x 2304 10.1 us, two ranges 8.3.)
+  if (f_pair < 0 && best.pair && best.bn == 64 && best.split == 1 && kblocks < 20)
+    best = evaluate(M, N, kblocks, sm_count, best.bn, 0, 1);
   fill_plan(M, N, kblocks, sm_count, forced, best, out);
   // What the caller's workspace must hold is decided by this plan. Running the ranges as clusters needs none, so a
   // cluster plan that is cheaper replaces it without asking for more.

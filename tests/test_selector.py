@@ -32,3 +32,20 @@ def test_plans(built_library, m, n, k):
     if p.split_k > 1:
         assert pkg.workspace_bytes(m, n, k) >= 4096 + (p.tiles - p.full_tiles) * p.split_k * 128 * p.block_n * 4 * (
             2 if p.cta_pair else 1)
+
+
+@pytest.mark.parametrize("m,n,k", [(1024, 1024, 1024), (300, 2000, 512), (200, 700, 1280)] + shapes(200, 2))
+def test_the_estimate_belongs_to_the_plan(built_library, m, n, k):
+    """64-wide single CTAs, no tile split: 400 clocks a K block and 1850 a tile, for every wave of tiles, and no cluster of the
+    same tiles would be cheaper by its own formula."""
+    p = pkg.describe(m, n, k)
+    if (m, n, k) == (1024, 1024, 1024):
+        assert (p.block_n, p.cta_pair, p.split_k) == (64, 0, 1)
+    if (p.block_n, p.cta_pair, p.split_k) != (64, 0, 1):
+        return
+    cost, kb = -(-p.tiles // 148) * (k // 128 * 400 + 1850), k // 128
+    assert pkg.estimate_clocks(m, n, k) == cost
+    for split, at_once in CLUSTERS.items():
+        if split * 2 <= kb and p.tiles <= at_once:
+            rows = min(m, 128) / 128
+            assert -(-kb // split) * 400 + 1850 + 2600 + 360 * split * (0.5 + 0.5 * rows) >= cost
