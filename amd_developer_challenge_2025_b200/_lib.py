@@ -1,17 +1,18 @@
 """ctypes binding of lib/libb200fp8mm.so (declarations: include/b200_fp8_mm.h, include/b200_mla_consumers.h), and the
 native module that makes the same calls for plain CUDA tensors without ctypes (csrc/host_calls.cpp).
 
-Loading fails loudly: there is no fallback implementation of the operator."""
+Loading the library fails loudly: there is no fallback implementation of the operator. The native module only checks and
+passes on arguments; without it the same is done in Python."""
 from __future__ import annotations
 
 import ctypes
 import importlib.util
 import os
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 # B200_FP8_MM_LIB selects another build of the same library (e.g. one made with extra nvcc flags).
 LIB_PATH = os.environ.get("B200_FP8_MM_LIB") or os.path.join(HERE, "lib", "libb200fp8mm.so")
-HOST_PATH = os.path.join(HERE, "lib", "_host.so")
 
 ABI_VERSION = 7
 
@@ -62,20 +63,34 @@ _lib = None
 _host = None
 
 
+class _PythonChecks:
+    """What stands in for the native module where it has not been built: every call goes through the checks in Python."""
+
+    @staticmethod
+    def fp8_mm(*args):
+        return False
+
+    fp8_mm_grouped = mla_decode = div_softmax = fp8_mm
+
+
 def host_calls():
-    """The native module lib/_host.so, bound to the loaded library. Its functions return False, having done nothing,
-    for whatever is not the plain case."""
+    """The native module, bound to the loaded library. Its functions return False, having done nothing, for whatever is not
+    the plain case."""
     return _host if _host is not None else _load_host()
 
 
 def _load_host():
     global _host
-    lib = load()
-    if not os.path.exists(HOST_PATH):
-        raise ImportError(f"{HOST_PATH} is missing: build it with `python -m amd_developer_challenge_2025_b200.build`.")
-    import torch  # noqa: F401  (the module's undefined symbols are torch's)
+    from .build import host_path
 
-    spec = importlib.util.spec_from_file_location("_host", HOST_PATH)
+    lib = load()
+    path = host_path()
+    if not os.path.exists(path):
+        warnings.warn(f"{path} is missing: calls are checked in Python, some 10 us each. Build it with "
+                      "`python -m amd_developer_challenge_2025_b200.build`.", RuntimeWarning, stacklevel=4)
+        _host = _PythonChecks
+        return _host
+    spec = importlib.util.spec_from_file_location("_host", path)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
     mod.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in

@@ -18,7 +18,16 @@ HEADERS = [os.path.join(INCLUDE, "b200_fp8_mm.h"), os.path.join(INCLUDE, "b200_m
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libb200fp8mm.so")
 HOST_SRC = os.path.join(HERE, "csrc", "host_calls.cpp")  # the entry points' per-call host work (a CPython module)
-HOST_LIB = os.path.join(LIB_DIR, "_host.so")
+
+
+def host_path() -> str:
+    """Where the native module for the running Python and torch lies. It is compiled against the internals of both, so both
+    are in its name and a module built for others is neither loaded nor taken for up to date."""
+    import sysconfig
+
+    import torch
+
+    return os.path.join(LIB_DIR, f"_host.{sysconfig.get_config_var('SOABI')}.torch-{torch.__version__}.so")
 
 
 def _nvcc() -> str:
@@ -31,7 +40,7 @@ def _outdated(target: str, sources) -> bool:
 
 
 def needs_build() -> bool:
-    return _outdated(LIB, SOURCES + HEADERS) or _outdated(HOST_LIB, [HOST_SRC] + HEADERS)
+    return _outdated(LIB, SOURCES + HEADERS) or _outdated(host_path(), [HOST_SRC] + HEADERS)
 
 
 def _build_host() -> None:
@@ -44,14 +53,14 @@ def _build_host() -> None:
     subprocess.check_call([
         os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{p}" for p in includes),
-        HOST_SRC, "-o", HOST_LIB, *(f"-L{p}" for p in library_paths()),
+        HOST_SRC, "-o", host_path(), *(f"-L{p}" for p in library_paths()),
         "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python",
     ])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(LIB_DIR, exist_ok=True)
-    if force or _outdated(HOST_LIB, [HOST_SRC] + HEADERS):
+    if force or _outdated(host_path(), [HOST_SRC] + HEADERS):
         _build_host()
     if not force and not _outdated(LIB, SOURCES + HEADERS):
         return LIB
