@@ -57,17 +57,19 @@ const at::Tensor* lookup(PyObject* dict, PyObject* key) {
   return v != nullptr ? plain_tensor(v) : nullptr;
 }
 
-// fp8_mm(a, b, a_scale, b_scale, c, n_phase, workspaces, status)
+// fp8_mm(a, b, a_scale, b_scale, c, n_phase, workspaces, status[, address of the forced b200_fp8_mm_plan or 0])
 bool run_fp8_mm(PyObject* const* args) {
   const at::Tensor *a = plain_tensor(args[0]), *b = plain_tensor(args[1]), *as = plain_tensor(args[2]),
                    *bs = plain_tensor(args[3]), *c = plain_tensor(args[4]);
-  if (!a || !b || !as || !bs || !c || !PyLong_CheckExact(args[5])) return false;
+  if (!a || !b || !as || !bs || !c || !PyIndex_Check(args[5])) return false;
   const c10::DeviceIndex dev = c10::cuda::current_device();
   if (!is_cuda(*a, at::kFloat8_e4m3fn, 2, dev) || !is_cuda(*b, at::kFloat8_e4m3fn, 2, dev) ||
       !is_cuda(*as, at::kFloat, 2, dev) || !is_cuda(*bs, at::kFloat, 2, dev) || !is_cuda(*c, at::kBFloat16, 2, dev))
     return false;
-  const long phase = PyLong_AsLong(args[5]);
+  const Py_ssize_t phase = PyNumber_AsSsize_t(args[5], nullptr);
   if (phase < 0 || phase >= kScaleBlock) return false;
+  const auto* plan = static_cast<const b200_fp8_mm_plan*>(args[8] != nullptr ? PyLong_AsVoidPtr(args[8]) : nullptr);
+  if (PyErr_Occurred()) return false;
   const int64_t m = a->size(0), k = a->size(1), n = b->size(0);
   if (m <= 0 || n <= 0 || k <= 0 || !fits_int(m) || !fits_int(n) || !fits_int(k) || k % kScaleBlock != 0) return false;
   const int64_t kb = k / kScaleBlock, nb = (n + phase + kScaleBlock - 1) / kScaleBlock;
@@ -90,7 +92,7 @@ bool run_fp8_mm(PyObject* const* args) {
                    static_cast<int>(k), a0, a1, b0, b1, as->stride(0), as->stride(1), bs->stride(0), bs->stride(1),
                    c->stride(0), static_cast<int>(phase), ws ? ws->data_ptr() : nullptr,
                    ws ? static_cast<size_t>(ws->numel()) : 0, static_cast<int*>(st->data_ptr()), stream,
-                  static_cast<const b200_fp8_mm_plan*>(nullptr));
+                  plan);
 }
 
 // fp8_mm_grouped(a, b, a_scale, b_scale, c, m_valid or None, status)
@@ -188,12 +190,15 @@ bool run_softmax(PyObject* const* args) {
 }
 
 // A C++ exception (a tensor without storage, a device that is gone) is "not the plain case" too.
-template <bool (*F)(PyObject* const*), Py_ssize_t N>
+// The last `Optional` of the N arguments may be left out (null).
+template <bool (*F)(PyObject* const*), Py_ssize_t N, Py_ssize_t Optional = 0>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   bool done = false;
-  if (nargs == N) {
+  if (nargs <= N && nargs >= N - Optional) {
+    PyObject* all[N] = {};
+    for (Py_ssize_t i = 0; i < nargs; ++i) all[i] = args[i];
     try {
-      done = F(args);
+      done = F(all);
     } catch (...) {
       done = false;
     }
@@ -230,7 +235,7 @@ PyCFunction fast() {
 
 PyMethodDef methods[] = {
     {"bind", fast<bind>(), METH_FASTCALL, nullptr},
-    {"fp8_mm", fast<entry<run_fp8_mm, 8>>(), METH_FASTCALL, nullptr},
+    {"fp8_mm", fast<entry<run_fp8_mm, 9, 1>>(), METH_FASTCALL, nullptr},
     {"fp8_mm_grouped", fast<entry<run_grouped, 7>>(), METH_FASTCALL, nullptr},
     {"mla_decode", fast<entry<run_rope, 12>>(), METH_FASTCALL, nullptr},
     {"div_softmax", fast<entry<run_softmax, 6>>(), METH_FASTCALL, nullptr},

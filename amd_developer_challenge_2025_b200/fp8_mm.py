@@ -141,7 +141,7 @@ def _validate(a, b, a_scale, b_scale, c, n_phase, plan):
     _check(c.stride(1) == 1, "c must have N contiguous")
     dev = a.device
     _check(all(t.device == dev for t in (b, a_scale, b_scale, c)), "tensors on different devices")
-    return workspace_bytes(m, n, k, plan), (plan.to_c() if plan is not None else None)
+    return workspace_bytes(m, n, k, plan)
 
 
 def fp8_mm(a, b, a_scale, b_scale, c, n_phase: int = 0, plan: Plan | None = None, check: bool = False):
@@ -154,19 +154,22 @@ def fp8_mm(a, b, a_scale, b_scale, c, n_phase: int = 0, plan: Plan | None = None
     row inside its 128-row scale block (0 unless b is a column shard of a larger matrix).
     `plan`: force tile parameters (sweeps/tests). `check`: synchronise and raise if a wait
     inside the kernel expired. Asynchronous otherwise, like the reference's launcher."""
-    if plan is None and not check and _lib.host_calls().fp8_mm(a, b, a_scale, b_scale, c, n_phase, _workspaces,
-                                                               _status):
+    cplan = plan.to_c() if plan is not None else None
+    if _lib.host_calls().fp8_mm(a, b, a_scale, b_scale, c, n_phase, _workspaces, _status,
+                                ctypes.addressof(cplan) if cplan is not None else 0):
+        if check:
+            check_device_status(a.device)
         return c
     # Not the plain case, or a call that will be refused: the same checks here, with their errors.
+    dev = a.device
+    if dev.type == "cuda" and dev.index != torch.cuda.current_device():
+        with torch.cuda.device(dev):
+            return fp8_mm(a, b, a_scale, b_scale, c, n_phase, plan, check)
     lib = _lib.load()
-    nbytes, cplan = _validate(a, b, a_scale, b_scale, c, n_phase, plan)
+    nbytes = _validate(a, b, a_scale, b_scale, c, n_phase, plan)
     sa, sb, sas, sbs, sc = a.stride(), b.stride(), a_scale.stride(), b_scale.stride(), c.stride()
     m, k = a.shape
     n = b.shape[0]
-    dev = a.device
-    if dev.index != torch.cuda.current_device():
-        with torch.cuda.device(dev):
-            return fp8_mm(a, b, a_scale, b_scale, c, n_phase, plan, check)
     stream = torch.cuda.current_stream(dev).cuda_stream
     ws = _workspace(dev, nbytes, stream)
     st = _status_words(dev)

@@ -13,13 +13,14 @@ from .fp8_mm import Fp8MmError, _check, fp8_mm
 
 
 def _check_range(name, t, off, d0, d1, d2, s1, s2):
-    """Every element off + i0*s1 + i1*s2 + j (strides of either sign) lies inside t's storage."""
-    spans = ((d0 - 1) * s1, (d1 - 1) * s2)
-    first = off + sum(min(0, v) for v in spans)
-    last = off + sum(max(0, v) for v in spans) + d2 - 1
-    start = t.storage_offset()
-    _check(0 <= off and 0 <= start + first and start + last < t.untyped_storage().nbytes() // t.element_size(),
-           f"{name}: range outside the tensor")
+    """Every element off + i0*s1 + i1*s2 + j (strides of either sign) lies inside the bf16 tensor's storage."""
+    first = last = off + t.storage_offset()
+    for span in ((d0 - 1) * s1, (d1 - 1) * s2):
+        if span < 0:
+            first += span
+        else:
+            last += span
+    _check(off >= 0 and first >= 0 and last + d2 <= t.untyped_storage().nbytes() // 2, f"{name}: range outside the tensor")
 
 
 def mla_decode(x, y, pos: int, xoff: int, yoff: int, d0: int, d1: int, d2: int, xs1: int, xs2: int, ys1: int,

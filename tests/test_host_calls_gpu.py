@@ -147,3 +147,19 @@ def test_integers_beyond_64_bits_launch_nothing(stubs, big):
     p = parts()
     assert not native.fp8_mm(*p, big, host._workspaces, host._status)
     assert stubs == []
+
+
+def test_forced_plans_and_checked_calls_are_native_too(stubs, monkeypatch):
+    """A plan reaches the library; a call that is to be checked is checked; a numpy n_phase is an integer. (The signature of
+    a forced plan used to be remembered; going through the Python checks each time took half as long again.)"""
+    import numpy as np
+    import amd_developer_challenge_2025_b200 as pkg
+    p, checked = parts(), []
+    monkeypatch.setattr(host, "check_device_status", checked.append)
+    monkeypatch.setattr(host, "_validate", lambda *a: pytest.fail("checked in Python"))
+    plan = host.Plan(block_n=64, cta_pair=-1, split_k=2, stages=4)
+    assert pkg.fp8_mm(*p, plan=plan) is p[4]
+    assert stubs[0][-1] and pkg.fp8_mm(*p) is p[4] and not stubs[1][-1]
+    assert pkg.fp8_mm(*p, n_phase=np.int64(96)) is p[4] and stubs[2][17] == 96
+    assert checked == [] and pkg.fp8_mm(*p, check=True) is p[4] and checked == [p[0].device]
+    assert len(stubs) == 4
