@@ -287,8 +287,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// One CTA per row. Pass 1 reads the row (16-byte loads between the row's first and last 16-byte boundary), forms e = expf(v * scale)
-// and the fp32 row sum; pass 2 reads the row again (it is in L1/L2 now), rounds e to bf16 as the reference keeps
+// One CTA per row, for rows that do not fit the registers. Pass 1 reads the row (16-byte loads between the row's first and
+// last 16-byte boundary), forms e = exp(v * scale) and the fp32 row sum; pass 2 reads the row again (it is in L1/L2 now), rounds e to bf16 as the reference keeps
 // it, divides by the sum and writes in place. HBM sees one read and one write of the row.
 __global__ void __launch_bounds__(kSoftmaxThreads) div_softmax_kernel(__nv_bfloat16* qk, int sl, float scale2) {
   __shared__ float scratch[kSoftmaxThreads / 32];
@@ -331,9 +331,6 @@ __global__ void __launch_bounds__(kSoftmaxThreads) div_softmax_kernel(__nv_bfloa
   }
 }
 
-// Longer rows, up to kRegRowElems elements (the reference's own limit is 8192): the row is read ONCE, its exponentials
-// stay in registers (as the bf16 values the reference keeps) across the block-wide sum, and the quotients are
-// written back; four independent 16-byte loads per thread are in flight at a time.
 // <<<grid, threads>>> on `stream`, allowed to begin under the kernel before it (see pdl_wait).
 template <typename... Params, typename... Args>
 int launch_pdl(void (*kernel)(Params...), dim3 grid, int threads, void* stream, Args... args) {
@@ -369,6 +366,9 @@ __device__ __forceinline__ float block_sum_256(float v, float* scratch) {
   return __shfl_sync(0xffffffffu, t, 0);
 }
 
+// Longer rows, up to kRegRowElems elements (the reference's own limit is 8192): the row is read ONCE, its exponentials
+// stay in registers (as the bf16 values the reference keeps) across the block-wide sum, and the quotients are
+// written back; four independent 16-byte loads per thread are in flight at a time.
 __global__ void __launch_bounds__(kRegThreads, 8) div_softmax_regs_kernel(__nv_bfloat16* qk, int sl, float scale2) {
   __shared__ float scratch[kRegThreads / 32];
   pdl_wait();
