@@ -1760,11 +1760,17 @@ int tmem_bufs_in_use(int block_n, int stages) {
   return d < stages ? d : stages;
 }
 
+// MMA-issuing threads (see the kernel).
+int issuers_for(int block_n) { return block_n <= 128 ? 2 : 1; }
+
 // Deepest ring that fits. The 256-wide tiles stop at four stages: a fifth measured 5 % slower (their
-// promotion warps still spill a little, and local memory loses L1 to every extra stage).
+// promotion warps still spill a little, and local memory loses L1 to every extra stage). Where two issuers share the
+// ring by stage, an odd one gives the first of them more K blocks and two in a row: 128-wide tiles with four stages for
+// five, 369 x 3196 x 1792 12.0 -> 11.8 us, 500 x 2385 x 4352 19.0 -> 18.5, 6763 x 624 x 1152 11.4 -> 11.0.
 int max_stages_for(int block_n, int pair, int store_bufs) {
   int s = block_n == 256 ? 4 : kMaxStages;
   while (s > 2 && smem_bytes_for(block_n, s, pair, store_bufs) > kMaxSmem) --s;
+  if (issuers_for(block_n) == 2 && s > 2 && s % 2 != 0) --s;
   return s;
 }
 
@@ -2226,7 +2232,7 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   kp.idesc_major = (a_mn ? (1u << 15) : 0u) | (b_mn ? (1u << 16) : 0u);
   // Two issuing threads pay off where the MMAs are short (narrow tiles: 25 % faster at block_n 64,
   // 10 % at 128); the wide tiles are bound by the promotion warps and run 1 % better with one.
-  kp.issuers = pl.block_n <= 128 ? 2 : 1;
+  kp.issuers = issuers_for(pl.block_n);
   {
     // Tile rows per raster group: the tiles running at one time form a block as square as possible.
     const int units = pl.cta_pair ? sm_count / 2 : sm_count;
@@ -2397,7 +2403,7 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.b_desc_lo = lb.desc_lo;
   kp.b_desc_hi = lb.desc_hi;
   kp.b_kstep = lb.kstep;
-  kp.issuers = pl.block_n <= 128 ? 2 : 1;
+  kp.issuers = issuers_for(pl.block_n);
   {
     const int units = pl.cta_pair ? sm_count / 2 : sm_count;
     int g = (units + kp.tiles_n / 2) / kp.tiles_n;

@@ -16,7 +16,7 @@
 // A stage has ONE issuer because a barrier wait tells only the parity of a phase: a thread that waits for use n of a stage
 // must have seen use n - 1 complete, or it takes "use n - 1 is still outstanding" for "use n is complete". With every second
 // block to each issuer, the stages of an odd ring change hands, and an issuer whose own blocks had landed first issued MMAs on
-// a stage whose copies were still in flight (128-wide tiles run five stages).
+// a stage whose copies were still in flight (128-wide tiles then ran five stages).
 struct IssuerWalk {
   int stage, buffer;
   uint32_t phase;

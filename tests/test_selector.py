@@ -49,3 +49,9 @@ def test_the_estimate_belongs_to_the_plan(built_library, m, n, k):
         if split * 2 <= kb and p.tiles <= at_once:
             rows = min(m, 128) / 128
             assert -(-kb // split) * 400 + 1850 + 2600 + 360 * split * (0.5 + 0.5 * rows) >= cost
+
+
+@pytest.mark.parametrize("m,n,k", [(369, 3196, 1792), (500, 2385, 4352)] + shapes(100, 3))
+def test_two_issuers_get_an_even_ring(built_library, m, n, k):
+    p = pkg.describe(m, n, k)
+    assert p.block_n > 128 or p.stages % 2 == 0
