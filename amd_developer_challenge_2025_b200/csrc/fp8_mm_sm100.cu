@@ -92,13 +92,11 @@ struct KernelParams {
   // 1 / (rows of the last, shorter raster group), 1 / split_k, 1 / (tiles_m * tiles_n), 1 / tiles_n.
   float rcp_per_group, rcp_raster, rcp_raster_last, rcp_split, rcp_per_problem, rcp_tiles_n;
   int b_scale_rows;
-  int vec_store;  // 1 when c, ldc and N allow 16-byte stores
   int stages;
   uint32_t stage_tx;  // bytes the copies of one K block bring to this CTA's stage
   int tmem_bufs;  // TMEM partial buffers in use: divides stages, at most TileCfg::kTmemBufs
   int issuers;     // MMA-issuing threads in use: 1 or 2
   int store_bufs;  // staging buffers per promotion warpgroup for the TMA store of c: 0 (plain stores), 1 .. 4
-  int row_stage_bufs;  // the same buffers where the TMA store cannot address c and tiles leave row by row; 0: no staging
   // Operand layout, as the values the producer and the MMA threads need (see OperandLayout below).
   int a_mn, b_mn;            // 1: the operand is MN-major in global and shared memory
   int b_boxes;               // TMA boxes per stage of b (1 when K-major)
@@ -464,6 +462,90 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
+}
+
+// One 32-byte sector.
+__device__ __forceinline__ void st_sector(void* dst, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
+// A thread's COLS fp32 values of one row as bf16 to dst, the first `cols` of them, at any 2-byte alignment, as whole
+// 32-byte sectors and the pieces of 1, 2, 4 and 8 elements that lead up to the first and follow the last.
+//
+// What bounds these stores is how many sectors are written in part: an L2 sector that is written in two halves costs far more
+// than two whole ones. The row's own distance to its first sector decides by how many elements everything has to move, so the
+// values go through a shifter of one, two, four and eight elements in registers; the leading pieces fall out of its stages.
+// 1000 x 4099 x 2304 (256-wide pairs; 1000 x 4104 through the TMA store takes 16.5 us): 24.9 us with rows written sixteen
+// lanes wide out of shared memory in 4-byte words, 17.2 us this way; 5947 x 7195 x 1024 164 -> 80, 46 x 1046 x 512 6.2 -> 4.2.
+template <int COLS>
+__device__ __forceinline__ void store_row(__nv_bfloat16* dst, int cols, const float2 (&acc)[COLS / 2]) {
+  if (cols <= 0) return;
+  constexpr int kWords = COLS / 2;
+  uint32_t w[kWords];
+#pragma unroll
+  for (int j = 0; j < kWords; ++j) w[j] = pack_bf16x2(acc[j].x, acc[j].y);
+  unsigned short* d = reinterpret_cast<unsigned short*>(dst);
+  if (cols < 16) {  // the end of a ragged matrix: less than a sector
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (2 * j < cols) d[2 * j] = static_cast<unsigned short>(w[j]);
+      if (2 * j + 1 < cols) d[2 * j + 1] = static_cast<unsigned short>(w[j] >> 16);
+    }
+    return;
+  }
+  const int head = static_cast<int>(-(reinterpret_cast<uintptr_t>(dst) >> 1)) & 15;  // elements up to the first sector
+  if (head & 1) {
+    *d = static_cast<unsigned short>(w[0]);
+    ++d;
+  }
+#pragma unroll
+  for (int j = 0; j < kWords; ++j) w[j] = (head & 1) ? __funnelshift_r(w[j], j + 1 < kWords ? w[j + 1] : 0u, 16) : w[j];
+  if (head & 2) {
+    *reinterpret_cast<uint32_t*>(d) = w[0];
+    d += 2;
+  }
+#pragma unroll
+  for (int j = 0; j < kWords; ++j) w[j] = (head & 2) ? (j + 1 < kWords ? w[j + 1] : 0u) : w[j];
+  if (head & 4) {
+    *reinterpret_cast<uint2*>(d) = make_uint2(w[0], w[1]);
+    d += 4;
+  }
+#pragma unroll
+  for (int j = 0; j < kWords; ++j) w[j] = (head & 4) ? (j + 2 < kWords ? w[j + 2] : 0u) : w[j];
+  if (head & 8) {
+    *reinterpret_cast<uint4*>(d) = make_uint4(w[0], w[1], w[2], w[3]);
+    d += 8;
+  }
+#pragma unroll
+  for (int j = 0; j < kWords; ++j) w[j] = (head & 8) ? (j + 4 < kWords ? w[j + 4] : 0u) : w[j];
+  const int left = cols - head;
+#pragma unroll
+  for (int k = 0; k < COLS / 16; ++k) {
+    uint32_t* v = w + 8 * k;
+    if (16 * k + 16 <= left) {
+      st_sector(d + 16 * k, v);
+    } else if (16 * k < left) {
+      unsigned short* e = d + 16 * k;
+      if (left & 8) {
+        *reinterpret_cast<uint4*>(e) = make_uint4(v[0], v[1], v[2], v[3]);
+        e += 8;
+      }
+      const uint32_t x0 = (left & 8) ? v[4] : v[0], x1 = (left & 8) ? v[5] : v[1];
+      const uint32_t x2 = (left & 8) ? v[6] : v[2], x3 = (left & 8) ? v[7] : v[3];
+      if (left & 4) {
+        *reinterpret_cast<uint2*>(e) = make_uint2(x0, x1);
+        e += 4;
+      }
+      const uint32_t y0 = (left & 4) ? x2 : x0, y1 = (left & 4) ? x3 : x1;
+      if (left & 2) {
+        *reinterpret_cast<uint32_t*>(e) = y0;
+        e += 2;
+      }
+      if (left & 1) *e = static_cast<unsigned short>((left & 2) ? y1 : y0);
+    }
+  }
 }
 
 // Shared-memory matrix descriptor (sm_100 format), as two 32-bit words.
@@ -1329,7 +1411,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       // The TMA store clips at the tensor's edges only: a tile that a group's row count cuts short goes out
       // through the guarded plain stores instead.
       const bool tma_rows_ok = MODE != kGrouped || (it.m_limit == p.M) || (it.m0 + Cfg::kTileM <= it.m_limit);
-      if (do_store && p.store_bufs > 0 && tma_rows_ok) {
+      if (__builtin_expect(do_store && p.store_bufs > 0 && tma_rows_ok, 1)) {
         // bf16 tile -> swizzled staging -> TMA store, 32 columns at a time per warpgroup. The
         // 16-byte piece q of row r sits at r*64 + ((q ^ ((r >> 1) & 3)) * 16) (SWIZZLE_64B), which
         // spreads a warp's stores over all banks.
@@ -1402,79 +1484,11 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             if (wg_tid == 0 && *abort_flag == 0) store_box(ch, bufi);
           }
         }
-      } else if (do_store && p.row_stage_bufs > 0) {
-        // Rows of c whose base or pitch is not 16-byte aligned: the warp stages 32 columns of its own 32 rows in shared
-        // memory and writes them out row by row, sixteen lanes to a row with one 4-byte word each. Left to the thread
-        // that owns a row, every store instruction touches 32 rows: 1000 x 4099 x 2304 took 53.2 us that way and takes
-        // 24.6 us this way.
-        constexpr int kBoxes = Cfg::kColsPerThread / kStoreBoxCols;
-        uint8_t* warp_stage = staging + half * p.row_stage_bufs * kStoreBufBytes + quarter * (32 * 64);
-        const int m_warp = row - lane;  // first row of this warp
-        const int rows = ok ? min(32, it.m_limit - m_warp) : 0;
-        const int sub = lane >> 4, word = lane & 15;
-        __nv_bfloat16* cwarp = p.c + static_cast<long long>(it.group) * p.c_g + static_cast<long long>(m_warp) * p.ldc;
-#pragma unroll
-        for (int ch = 0; ch < kBoxes; ++ch) {
-          uint8_t* rowp = warp_stage + lane * 64;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int j = ch * 16 + q * 4;
-            uint4 o;
-            o.x = pack_bf16x2(acc[j + 0].x, acc[j + 0].y);
-            o.y = pack_bf16x2(acc[j + 1].x, acc[j + 1].y);
-            o.z = pack_bf16x2(acc[j + 2].x, acc[j + 2].y);
-            o.w = pack_bf16x2(acc[j + 3].x, acc[j + 3].y);
-            *reinterpret_cast<uint4*>(rowp + ((q ^ ((lane >> 1) & 3)) << 4)) = o;
-          }
-          __syncwarp();
-          const int cols = min(kStoreBoxCols, p.N - (col0 + ch * kStoreBoxCols));  // columns of this box that exist
-#pragma unroll 4
-          for (int i = 0; i < 16; ++i) {
-            const int r = 2 * i + sub;
-            __nv_bfloat16* dst = cwarp + static_cast<long long>(r) * p.ldc + col0 + ch * kStoreBoxCols;
-            // Word w of the staged row (elements 2w, 2w + 1). A row that starts between two words of global memory
-            // (odd) is written as elements 2w - 1 and 2w, the former from the lane before; element 31 is then left over.
-            const uint32_t cur = *reinterpret_cast<const uint32_t*>(
-                warp_stage + r * 64 + ((((word >> 2) ^ ((r >> 1) & 3)) << 4) | ((word & 3) << 2)));
-            const uint32_t before = __shfl_up_sync(0xffffffffu, cur, 1, 16);
-            const bool odd = ((reinterpret_cast<uintptr_t>(dst) >> 1) & 1u) != 0;
-            const int e0 = 2 * word - (odd ? 1 : 0);
-            const uint32_t two = odd ? __funnelshift_r(before, cur, 16) : cur;
-            if (r < rows) {
-              if (e0 >= 0 && e0 + 1 < cols) {
-                *reinterpret_cast<uint32_t*>(dst + e0) = two;
-              } else {
-                if (e0 >= 0 && e0 < cols) *reinterpret_cast<unsigned short*>(dst + e0) = static_cast<unsigned short>(two);
-                if (e0 < 0 && cols > 0) *reinterpret_cast<unsigned short*>(dst) = static_cast<unsigned short>(cur);
-              }
-              if (odd && word == 15 && cols == kStoreBoxCols)
-                *reinterpret_cast<unsigned short*>(dst + 31) = static_cast<unsigned short>(cur >> 16);
-            }
-          }
-          __syncwarp();
-        }
       } else if (do_store && ok) {
-        if (row < it.m_limit) {
-          __nv_bfloat16* crow = p.c + static_cast<long long>(it.group) * p.c_g + static_cast<long long>(row) * p.ldc;
-#pragma unroll
-          for (int j = 0; j < Cfg::kColsPerThread / 8; ++j) {
-            const int col = col0 + j * 8;
-            if (p.vec_store && col + 8 <= p.N) {
-              uint4 o;
-              o.x = pack_bf16x2(acc[j * 4 + 0].x, acc[j * 4 + 0].y);
-              o.y = pack_bf16x2(acc[j * 4 + 1].x, acc[j * 4 + 1].y);
-              o.z = pack_bf16x2(acc[j * 4 + 2].x, acc[j * 4 + 2].y);
-              o.w = pack_bf16x2(acc[j * 4 + 3].x, acc[j * 4 + 3].y);
-              *reinterpret_cast<uint4*>(crow + col) = o;
-            } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                if (col + 2 * e < p.N) crow[col + 2 * e] = __float2bfloat16_rn(acc[j * 4 + e].x);
-                if (col + 2 * e + 1 < p.N) crow[col + 2 * e + 1] = __float2bfloat16_rn(acc[j * 4 + e].y);
-              }
-            }
-          }
-        }
+        const int at = it.m0 + static_cast<int>(cta_rank) * kBlockM + quarter * 32 + lane;
+        if (at < it.m_limit)
+          store_row<Cfg::kColsPerThread>(p.c + static_cast<long long>(it.group) * p.c_g + static_cast<long long>(at) * p.ldc + col0,
+                                         min(Cfg::kColsPerThread, p.N - col0), acc);
       }
     }
   }
@@ -1494,10 +1508,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       constexpr int kPieces = BN / 4;  // per row
       const int rows = min(kBlockM, p.M - it.m0);
       const uint32_t base = smem_u32(ring);
-      for (int u = it.split * Cfg::kEpiThreads + static_cast<int>(threadIdx.x) - 128; u < rows * kPieces;
-           u += ranges * Cfg::kEpiThreads) {
-        const int r = u / kPieces, col = (u % kPieces) * 4;
-        const uint32_t at = base + static_cast<uint32_t>(r * (BN + 4) + col) * 4u;
+      const int first = it.split * Cfg::kEpiThreads + static_cast<int>(threadIdx.x) - 128, step = ranges * Cfg::kEpiThreads;
+      auto piece_of = [&](int u) { return p.c + static_cast<long long>(it.m0 + u / kPieces) * p.ldc + it.n0 + (u % kPieces) * 4; };
+      auto reduced = [&](int u, uint32_t& lo, uint32_t& hi) {
+        const uint32_t at = base + static_cast<uint32_t>((u / kPieces) * (BN + 4) + (u % kPieces) * 4) * 4u;
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
         float4 t[kMaxCluster];
 #pragma unroll
@@ -1511,17 +1525,55 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             sum.z += t[s].z;
             sum.w += t[s].w;
           }
-        __nv_bfloat16* dst = p.c + static_cast<long long>(it.m0 + r) * p.ldc + it.n0 + col;
-        const int cols = p.N - (it.n0 + col);
-        const uint32_t lo = pack_bf16x2(sum.x, sum.y), hi = pack_bf16x2(sum.z, sum.w);
-        if (cols >= 4 && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
-          *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
-        } else {
-          unsigned short* d16 = reinterpret_cast<unsigned short*>(dst);
-          if (cols > 0) d16[0] = static_cast<unsigned short>(lo);
-          if (cols > 1) d16[1] = static_cast<unsigned short>(lo >> 16);
-          if (cols > 2) d16[2] = static_cast<unsigned short>(hi);
-          if (cols > 3) d16[3] = static_cast<unsigned short>(hi >> 16);
+        lo = pack_bf16x2(sum.x, sum.y);
+        hi = pack_bf16x2(sum.z, sum.w);
+      };
+      if (__builtin_expect(((reinterpret_cast<uintptr_t>(p.c) | static_cast<uintptr_t>(2 * p.ldc)) & 7) == 0, 1)) {
+        for (int u = first; u < rows * kPieces; u += step) {
+          uint32_t lo, hi;
+          reduced(u, lo, hi);
+          __nv_bfloat16* dst = piece_of(u);
+          const int cols = p.N - (it.n0 + (u % kPieces) * 4);
+          if (cols >= 4) {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
+          } else {
+            unsigned short* d16 = reinterpret_cast<unsigned short*>(dst);
+            if (cols > 0) d16[0] = static_cast<unsigned short>(lo);
+            if (cols > 1) d16[1] = static_cast<unsigned short>(lo >> 16);
+            if (cols > 2) d16[2] = static_cast<unsigned short>(hi);
+          }
+        }
+      } else {
+        // A row leaves in 8-byte pieces at whatever 8-byte boundaries it has in memory: a lane's piece starts at its
+        // element `skip` and ends in the next lane's elements. The ends of the row are written element by element. (Beside
+        // the loop above and not in it: its few instructions more cost 128 x 576 x 7168 0.2 of 7.8 us.)
+        for (int u = first; u - lane < rows * kPieces; u += step) {
+          const bool mine = u < rows * kPieces;  // the same for all kPieces lanes of a row
+          uint32_t lo = 0, hi = 0;
+          if (mine) reduced(u, lo, hi);
+          const uint32_t next_lo = __shfl_down_sync(0xffffffffu, lo, 1), next_hi = __shfl_down_sync(0xffffffffu, hi, 1);
+          unsigned short* d16 = reinterpret_cast<unsigned short*>(piece_of(u));
+          const int skip = static_cast<int>(-(reinterpret_cast<uintptr_t>(d16) >> 1)) & 3;
+          const uint32_t x0 = (skip & 2) ? hi : lo, x1 = (skip & 2) ? next_lo : hi, x2 = (skip & 2) ? next_hi : next_lo;
+          const uint32_t y0 = (skip & 1) ? __funnelshift_r(x0, x1, 16) : x0, y1 = (skip & 1) ? __funnelshift_r(x1, x2, 16) : x1;
+          if (mine) {
+            const int col = (u % kPieces) * 4;
+            const int cols = p.N - (it.n0 + col);  // from this lane's first element on
+            const int count = (col + 4 == BN ? min(cols, 4) : min(cols, 4 + skip)) - skip;
+            if (count == 4) {
+              *reinterpret_cast<uint2*>(d16 + skip) = make_uint2(y0, y1);
+            } else {
+              if (count > 0) d16[skip] = static_cast<unsigned short>(y0);
+              if (count > 1) d16[skip + 1] = static_cast<unsigned short>(y0 >> 16);
+              if (count > 2) d16[skip + 2] = static_cast<unsigned short>(y1);
+            }
+            if (col == 0) {
+              const int lead = min(skip, cols);
+              if (lead > 0) d16[0] = static_cast<unsigned short>(lo);
+              if (lead > 1) d16[1] = static_cast<unsigned short>(lo >> 16);
+              if (lead > 2) d16[2] = static_cast<unsigned short>(hi);
+            }
+          }
         }
       }
     }
@@ -2217,7 +2269,6 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   kp.stage_tx = static_cast<uint32_t>((a_box + b_box_rows_for(pl.block_n, pl.cta_pair)) * kBlockK);
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
   kp.store_bufs = store_bufs;
-  kp.row_stage_bufs = (reinterpret_cast<uintptr_t>(c) % 16) != 0 || (ldc % 8) != 0 ? pl.store_bufs : 0;
   kp.a_mn = a_mn ? 1 : 0;
   kp.b_mn = b_mn ? 1 : 0;
   kp.b_boxes = lb.boxes;
@@ -2243,8 +2294,6 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   }
   set_decode_reciprocals(kp);
   kp.b_scale_rows = ceil_div(N + n_phase, 128);
-  kp.vec_store =
-      ((reinterpret_cast<uintptr_t>(c) % 16) == 0 && (ldc % 8) == 0 && (N % 8) == 0) ? 1 : 0;
   kp.wait_limit_ns = opts.wait_limit_ns;
   kp.selftest_skip_kblock = opts.selftest_skip_kblock;
 
@@ -2391,9 +2440,6 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.stage_tx = static_cast<uint32_t>((a_box + b_rows_per_cta) * kBlockK);
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
   kp.store_bufs = store_bufs;
-  // (a tile that a group's row count cuts short leaves in 16-byte pieces where c allows them: 17 x 340 x 2304 x 384
-  // with uneven loads 23.9 us, staged row by row 32.0)
-  kp.row_stage_bufs = store_bufs == 0 ? pl.store_bufs : 0;
   kp.b_boxes = lb.boxes;
   kp.b_box_cols = lb.box_cols;
   kp.b_box_bytes = lb.box_bytes;
@@ -2413,7 +2459,6 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   }
   set_decode_reciprocals(kp);
   kp.b_scale_rows = ceil_div(N, 128);
-  kp.vec_store = ((reinterpret_cast<uintptr_t>(c) % 16) == 0 && (ldc % 8) == 0 && (c_g % 8) == 0 && (N % 8) == 0) ? 1 : 0;
   kp.wait_limit_ns = kWaitLimitNs;
   kp.selftest_skip_kblock = -1;
   kp.groups = groups;
