@@ -1775,6 +1775,13 @@ bool encode_output_map_3d(CUtensorMap* map, void* base, int groups, int M, int N
   return encode_map(map, k);
 }
 
+// Whether c can leave through the TMA store: base, row pitch and group pitch on 16-byte boundaries, and rows of whole 16 bytes,
+// because the store writes the last 16 bytes of a row in full: what lay behind a shorter row in a wider matrix was overwritten
+// (up to seven elements, with zeros). Other rows are written by store_row.
+bool tma_store_fits(const void* c, int N, long long ldc, long long c_g) {
+  return (reinterpret_cast<uintptr_t>(c) % 16) == 0 && (ldc % 8) == 0 && (c_g % 8) == 0 && (N % 8) == 0;
+}
+
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Rows of b per TMA box of one CTA (K-major b): a CTA of a pair loads half of the tile's rows.
@@ -2229,9 +2236,7 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   if (fn == nullptr) return B200_FP8_MM_ERR_PLAN;
 
   CUtensorMap map_a, map_b, map_c;
-  // The TMA store of c needs a 16-byte aligned base and row pitch; otherwise plain stores are used.
-  int store_bufs = pl.store_bufs;
-  if ((reinterpret_cast<uintptr_t>(c) % 16) != 0 || (ldc % 8) != 0) store_bufs = 0;
+  int store_bufs = tma_store_fits(c, N, ldc, 0) ? pl.store_bufs : 0;
   if (store_bufs > 0) {
     if (!encode_output_map(&map_c, c, M, N, ldc)) return B200_FP8_MM_ERR_DRIVER;
   } else {
@@ -2403,8 +2408,7 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   if (fn == nullptr) return B200_FP8_MM_ERR_PLAN;
 
   CUtensorMap map_a, map_b, map_c;
-  int store_bufs = pl.store_bufs;
-  if ((reinterpret_cast<uintptr_t>(c) % 16) != 0 || (ldc % 8) != 0 || (c_g % 8) != 0) store_bufs = 0;
+  int store_bufs = tma_store_fits(c, N, ldc, c_g) ? pl.store_bufs : 0;
   if (store_bufs > 0) {
     if (!encode_output_map_3d(&map_c, c, groups, M, N, ldc, c_g)) return B200_FP8_MM_ERR_DRIVER;
   } else {

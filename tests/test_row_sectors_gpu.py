@@ -32,7 +32,7 @@ def test_every_distance_to_a_sector(plan, n):
     a, b, a_s, b_s, _ = pkg.make_inputs(m, n, k, seed=n, device="cuda")
     aligned = torch.zeros(m, (n + 15) // 8 * 8, dtype=torch.bfloat16, device="cuda")
     fp8_mm(a, b, a_s, b_s, aligned[:, :n], plan=plan)
-    for pitch, offset in ((n | 1, 0), (n + 3 - n % 2, 5), ((n + 1) // 2 * 2, 2)):
+    for pitch, offset in ((n | 1, 0), (n + 3 - n % 2, 5), ((n + 1) // 2 * 2, 2), ((n + 7) // 8 * 8 + 8, 8)):
         buf, c = rows_in_a_guarded_buffer(m, n, pitch, offset)
         fp8_mm(a, b, a_s, b_s, c, plan=plan)
         check_device_status()
