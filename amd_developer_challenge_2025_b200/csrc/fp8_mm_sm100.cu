@@ -11,6 +11,7 @@
 // Structure of one CTA (384 threads, one CTA per SM, persistent over work items):
 //   warp 0      TMA producer: A (128 x 128 B) and B tiles of one K block into a SWIZZLE_128B
 //               shared-memory ring, completion on an mbarrier per stage
+//               (64-wide tiles: of two K blocks per stage, see stage_blocks_for)
 //   warp 1      MMA issuer: 4 x tcgen05.mma.kind::f8f6f4 (K=32 each) per K block into one of
 //               the TMEM partial buffers, then ONE tcgen05.commit to the stage's "done" barrier,
 //               which both frees the stage for the producer and publishes the buffer to the
@@ -18,8 +19,8 @@
 //               collects the promotion warps' release of the TMEM buffer that K block will
 //               overwrite (K block j uses stage j mod stages and buffer j mod buffers; a warp that
 //               has drained the buffer of K block j arrives on the barrier of K block j + buffers)
-//   warp 2      allocates / frees TMEM; its first lane is a second MMA issuer (the two issuers share
-//               the K blocks by ring stage, see issuer_walk.h)
+//   warp 2      allocates / frees TMEM; its first lane is a second MMA issuer at the narrow tiles (the
+//               two issuers take one K block each of a stage of two, or share the ring by stage, see issuer_walk.h)
 //   warp 3      scale loader: cp.async of the a_scale / b_scale values of FOUR K blocks at a time
 //               into a small shared-memory ring, up to 16 K blocks ahead
 //   warps 4-11  promotion + store: tcgen05.ld the partial, fma into register accumulators with
@@ -73,6 +74,18 @@ constexpr int kScaleGroup = 4;  // K blocks per scale-ring slot (4 or 8; 8 measu
 constexpr int kScaleSlots = 4;                                   // ring depth (16 K blocks)
 constexpr int kScaleSlotFloats = kBlockM * kScaleGroup + 4 * kScaleGroup;  // a[128][4] + b[4][4]
 constexpr int kBarrierBytes = 512;                                         // mbarriers and flags
+// MMA-issuing threads. Two pay off where the MMAs are short (narrow tiles: 25 % faster at 64 columns, 10 % at 128); the wide
+// tiles are bound by the promotion warps and run 1 % better with one.
+__host__ __device__ constexpr int issuers_for(int block_n) { return block_n <= 128 ? 2 : 1; }
+// K blocks per ring stage. A K block of a 64-wide tile is over sooner than the single-thread roles and the promotion warps get
+// through its barriers and copies (the producer needs about 420 clocks for its wait, expect_tx and two copies; the tensor core
+// 136, the operands' way into shared memory 390), so two of them share a stage: one wait, one expect_tx and two copies of the
+// producer, one wait and one release of the promotion warps for both. 2048 x 576 x 7168 18.1 -> 15.3 us, 32 x 576 x 1024 4.8 ->
+// 4.5. At 128 columns it was slower (8192 x 4608 x 7168 298 -> 304 us with single CTAs, 281 -> 280 with pairs; split in
+// clusters 256 x 1536 x 7168 11.2 -> 12.8): half as many stages fit, and the operands' way is what bounds it.
+__host__ __device__ constexpr int stage_blocks_for(int block_n) { return block_n == 64 ? 2 : 1; }
+// TMEM partial buffers, each for the K blocks of one stage (at most 512 columns in all).
+__host__ __device__ constexpr int tmem_bufs_for(int block_n) { return block_n <= 128 ? 4 : 2; }
 constexpr int kHeaderBytes = ((kBarrierBytes + kScaleSlots * kScaleSlotFloats * 4 + 1023) / 1024) * 1024;
 
 struct KernelParams {
@@ -92,10 +105,10 @@ struct KernelParams {
   // 1 / (rows of the last, shorter raster group), 1 / split_k, 1 / (tiles_m * tiles_n), 1 / tiles_n.
   float rcp_per_group, rcp_raster, rcp_raster_last, rcp_split, rcp_per_problem, rcp_tiles_n;
   int b_scale_rows;
-  int stages;
-  uint32_t stage_tx;  // bytes the copies of one K block bring to this CTA's stage
-  int tmem_bufs;  // TMEM partial buffers in use: divides stages, at most TileCfg::kTmemBufs
-  int issuers;     // MMA-issuing threads in use: 1 or 2
+  int stages;              // of TileCfg::kStageBlocks K blocks each
+  uint32_t stage_tx;       // bytes the copies of one stage bring to this CTA
+  uint32_t a_block_bytes;  // from one K block of a stage's a to the next
+  int tmem_bufs;  // TMEM partial buffers in use, each for a stage's K blocks: at most stages and TileCfg::kTmemBufs
   int store_bufs;  // staging buffers per promotion warpgroup for the TMA store of c: 0 (plain stores), 1 .. 4
   // Operand layout, as the values the producer and the MMA threads need (see OperandLayout below).
   int a_mn, b_mn;            // 1: the operand is MN-major in global and shared memory
@@ -277,6 +290,24 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
             dst),
         "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+  }
+}
+
+// And the form for grouped launches whose copies bring several K blocks.
+template <bool PAIR>
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+  if constexpr (PAIR) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+        : "memory");
+  } else {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+            dst),
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
         : "memory");
   }
 }
@@ -596,11 +627,13 @@ template <int BN, bool PAIR>
 struct TileCfg {
   static constexpr int kTileM = PAIR ? 2 * kBlockM : kBlockM;  // rows of C per tile
   static constexpr int kRowsB = PAIR ? BN / 2 : BN;            // rows of B this CTA loads per stage
-  static constexpr int kStageBytesA = kBlockM * kBlockK;
-  static constexpr int kStageBytesB = kRowsB * kBlockK;
-  static constexpr int kStageBytes = kStageBytesA + kStageBytesB;
-  static constexpr int kTmemBufs = (BN <= 128) ? 4 : 2;
-  static constexpr int kTmemColsUsed = kTmemBufs * BN;
+  static constexpr int kStageBlocks = stage_blocks_for(BN);  // K blocks that share a ring stage, its barriers and its copies
+  static constexpr int kBlockBytesB = kRowsB * kBlockK;
+  static constexpr int kStageBytesA = kStageBlocks * kBlockM * kBlockK;
+  static constexpr int kStageBytes = kStageBytesA + kStageBlocks * kBlockBytesB;
+  static constexpr int kTmemBufs = tmem_bufs_for(BN);
+  static constexpr int kTmemColsUsed = kTmemBufs * kStageBlocks * BN;
+  static constexpr int kIssuers = issuers_for(BN);
   static constexpr int kTmemCols = kTmemColsUsed <= 256 ? 256 : 512;  // power of two >= 32
   // Promotion warps: groups of four (one per TMEM lane quarter), each group owning a share of the
   // tile's columns. Two groups everywhere: a third group for the 192-wide tile (64 columns per
@@ -626,6 +659,7 @@ struct TileCfg {
   // 32-column fetches in flight with two landing areas was measured 5-8 % slower than one at a time.
   static constexpr int kChunkCols = (kColsPerThread == 64 || kWideLanding) ? 64 : 32;
   static constexpr int kChunks = kColsPerThread / kChunkCols;
+  static_assert(kStageBlocks == 1 || kChunks == 1, "a thread takes its whole share of each K block of a stage at once");
   // Accumulators as packed pairs (fma.rn.f32x2: half the issue slots) or as scalars. With 128 columns per
   // thread the packed form spills (the pairs want aligned 64-bit registers next to a 32-register landing
   // area); scalars fit, and the 256-wide pair plan went from 442 to 262 us on the headline GEMM.
@@ -863,7 +897,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
     for (int s = 0; s < kMaxStages; ++s) {
       // one arrive.expect_tx per producing CTA + one release per promotion warp (of both CTAs)
       mbar_init(smem_u32(&full_bar[s]), (PAIR ? 2 : 1) * (1 + Cfg::kEpiWarps));
-      mbar_init(smem_u32(&done_bar[s]), 1);  // the MMA thread's commit
+      mbar_init(smem_u32(&done_bar[s]), Cfg::kStageBlocks);  // a commit per K block
     }
     for (int s = 0; s < kScaleSlots; ++s) {
       mbar_init(smem_u32(&scale_full_bar[s]), 32);
@@ -995,13 +1029,14 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           if (MODE == kGrouped && it.done) break;
           const int a_row = it.m0 + static_cast<int>(cta_rank) * kBlockM;
           const int b_row = it.n0 + static_cast<int>(cta_rank) * (PAIR ? Cfg::kRowsB : 0);
-          for (int kb = it.kb_begin; kb < it.kb_end; ++kb) {
+          for (int kb = it.kb_begin; kb < it.kb_end; kb += Cfg::kStageBlocks) {
             if (!mbar_wait(smem_u32(&done_bar[stage]), phase ^ 1u, ctx, 0x100 | stage)) {
               ok = false;
               break;
             }
             if constexpr (BN == 64 && !PAIR && MODE == kPlain) {
-              if (kb == p.selftest_skip_kblock && w == work_begin()) {  // self-test only: this block never arrives
+              // self-test only: the stage with this block never arrives
+              if (p.selftest_skip_kblock >= kb && p.selftest_skip_kblock < kb + Cfg::kStageBlocks && w == work_begin()) {
                 if (++stage == stages) {
                   stage = 0;
                   phase ^= 1u;
@@ -1009,35 +1044,41 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
                 continue;
               }
             }
-            // Both CTAs of a pair report to the leader's barrier: its MMA thread consumes the stage.
+            // Both CTAs of a pair report to the leader's barrier: its MMA threads consume the stage.
             const uint32_t fb = PAIR ? map_to_cta(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
-#ifdef FP8MM_X_NOTMA
-            mbar_expect_tx_cluster(fb, 0);
-            if (++stage == stages) {
-              stage = 0;
-              phase ^= 1u;
-            }
-            continue;
-#endif
             mbar_expect_tx_cluster(fb, p.stage_tx);
             const uint32_t sa = smem_u32(ring + stage * Cfg::kStageBytes);
-            // K-major: x = byte of K, y = matrix row. MN-major: x = matrix row (a multiple of 64), y = k.
-            if (MODE == kGrouped) {
-              tma_load_3d<PAIR>(sa, &tmap_a, kb * kBlockK, a_row, it.group, fb);
-              tma_load_3d<PAIR>(sa + Cfg::kStageBytesA, &tmap_b, kb * kBlockK, b_row, it.group, fb);
+            const uint32_t sb = sa + Cfg::kStageBytesA;
+            // K-major: x = byte of K, y = matrix row; where a stage has several K blocks, x = byte of a block, y = row,
+            // z = block. MN-major: x = matrix row (a multiple of 64), y = k. K blocks past the end of K arrive as zeros.
+            if constexpr (MODE == kGrouped) {
+              if constexpr (Cfg::kStageBlocks > 1) {
+                tma_load_4d<PAIR>(sa, &tmap_a, 0, a_row, kb, it.group, fb);
+                tma_load_4d<PAIR>(sb, &tmap_b, 0, b_row, kb, it.group, fb);
+              } else {
+                tma_load_3d<PAIR>(sa, &tmap_a, kb * kBlockK, a_row, it.group, fb);
+                tma_load_3d<PAIR>(sb, &tmap_b, kb * kBlockK, b_row, it.group, fb);
+              }
             } else {
-            if (MODE != kMnMajor || !p.a_mn) {
-              tma_load_2d<PAIR>(sa, &tmap_a, kb * kBlockK, a_row, fb);
-            } else {
-              tma_load_2d<PAIR>(sa, &tmap_a, a_row, kb * kBlockK, fb);
-            }
-            if (MODE != kMnMajor || !p.b_mn) {
-              tma_load_2d<PAIR>(sa + Cfg::kStageBytesA, &tmap_b, kb * kBlockK, b_row, fb);
-            } else {
-              for (int i = 0; i < p.b_boxes; ++i)
-                tma_load_2d<PAIR>(sa + Cfg::kStageBytesA + static_cast<uint32_t>(i * p.b_box_bytes), &tmap_b,
-                                  b_row + i * p.b_box_cols, kb * kBlockK, fb);
-            }
+              auto load_k_major = [&](uint32_t dst, const CUtensorMap* map, int row) {
+                if constexpr (Cfg::kStageBlocks > 1) {
+                  tma_load_3d<PAIR>(dst, map, 0, row, kb, fb);
+                } else {
+                  tma_load_2d<PAIR>(dst, map, kb * kBlockK, row, fb);
+                }
+              };
+              if (MODE != kMnMajor || !p.a_mn) {
+                load_k_major(sa, &tmap_a, a_row);
+              } else {
+                tma_load_2d<PAIR>(sa, &tmap_a, a_row, kb * kBlockK, fb);
+              }
+              if (MODE != kMnMajor || !p.b_mn) {
+                load_k_major(sb, &tmap_b, b_row);
+              } else {
+                for (int i = 0; i < p.b_boxes; ++i)
+                  tma_load_2d<PAIR>(sb + static_cast<uint32_t>(i * p.b_box_bytes), &tmap_b, b_row + i * p.b_box_cols,
+                                    kb * kBlockK, fb);
+              }
             }
             if (++stage == stages) {
               stage = 0;
@@ -1055,51 +1096,55 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       __syncwarp();
     } else if (warp == 1 || warp == 2) {
       // ---------------- MMA issuers (the leader CTA of a pair issues for both) ----------------
-      // Up to two threads, one in each warp, share the K blocks by ring stage. A K block's MMAs go to a TMEM
-      // buffer of their own, so the two streams need no ordering between them; one thread alone spends
+      // Up to two threads, one in each warp, share the K blocks: one of each stage's two, or every second stage. A K block's
+      // MMAs go to TMEM columns of their own, so the two streams need no ordering between them; one thread alone spends
       // about 700 clocks per K block on its barrier wait and on issuing (an MMA costs the issuing
       // thread roughly 100 clocks), more than the tensor pipe needs for a narrow tile's block.
-      if (lane == 0 && cta_rank == 0 && warp - 1 < p.issuers) {
+      if (lane == 0 && cta_rank == 0 && warp - 1 < Cfg::kIssuers) {
         constexpr uint32_t kHiK = (1024u >> 4) | (1u << 14) | (2u << 29);  // K-major, 128-byte swizzle
         const uint32_t idesc = make_idesc(Cfg::kTileM, BN) | (MODE == kMnMajor ? p.idesc_major : 0u);
         const uint32_t a_hi = MODE == kMnMajor ? p.a_desc_hi : kHiK, b_hi = MODE == kMnMajor ? p.b_desc_hi : kHiK;
         const uint32_t a_kstep = MODE == kMnMajor ? p.a_kstep : 2u, b_kstep = MODE == kMnMajor ? p.b_kstep : 2u;
         const uint32_t a_lo_bits = MODE == kMnMajor ? p.a_desc_lo : (1u << 16), b_lo_bits = MODE == kMnMajor ? p.b_desc_lo : (1u << 16);
         const int me = warp - 1;
+        constexpr bool kShared = Cfg::kStageBlocks > 1;  // the issuers share every stage
+        const int my_block = kShared ? me : 0;           // of a stage
         const int total_work = work_total(), work_step = work_stride();
-        const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_base_slot);
-        // Each issuer visits only its own K blocks (see IssuerWalk, which runs on across tile boundaries) and keeps
-        // its ring position with add-and-wrap only: no division and no work for the other issuer's blocks on this
+        const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_base_slot) + static_cast<uint32_t>(my_block * BN);
+        const uint32_t a_base = smem_u32(ring) + static_cast<uint32_t>(my_block) * p.a_block_bytes;
+        const uint32_t b_base = smem_u32(ring) + Cfg::kStageBytesA + static_cast<uint32_t>(my_block * Cfg::kBlockBytesB);
+        // Each issuer visits only its own stages (see IssuerWalk, which runs on across tile boundaries) and keeps
+        // its ring position with add-and-wrap only: no division and no work for the other issuer's stages on this
         // thread, whose scalar instructions are on the critical path.
         IssuerWalk at;
-        at.begin(me, stages, nbufs);
+        at.begin(kShared ? 0 : me, stages, nbufs);
         bool ok = true;
         for (int w = work_begin(); w < total_work && ok; w += work_step) {
           const WorkItem it = work_item(w);
           if (MODE == kGrouped && it.done) break;
           const int blocks = it.kb_end - it.kb_begin;
-          while (at.block < blocks) {
-            const uint32_t sa = smem_u32(ring + at.stage * Cfg::kStageBytes);
-            const uint32_t a_lo = smem_desc_addr(sa) | a_lo_bits;
-            const uint32_t b_lo = smem_desc_addr(sa + Cfg::kStageBytesA) | b_lo_bits;
-            const uint32_t d_addr = tmem_base + static_cast<uint32_t>(at.buffer * BN);
-            // operands landed AND the TMEM buffer of this K block drained (see the promotion warps)
+          const int uses = (blocks + Cfg::kStageBlocks - 1) / Cfg::kStageBlocks;
+          while (at.block < uses) {
+            const uint32_t a_lo = smem_desc_addr(a_base + static_cast<uint32_t>(at.stage * Cfg::kStageBytes)) | a_lo_bits;
+            const uint32_t b_lo = smem_desc_addr(b_base + static_cast<uint32_t>(at.stage * Cfg::kStageBytes)) | b_lo_bits;
+            const uint32_t d_addr = tmem_base + static_cast<uint32_t>(at.buffer * Cfg::kStageBlocks * BN);
+            // operands landed AND the TMEM buffer of this stage drained (see the promotion warps)
             if (!mbar_wait(smem_u32(&full_bar[at.stage]), at.phase, ctx, 0x300 | at.stage)) {
               ok = false;
               break;
             }
             tcgen05_fence_after();
-#ifndef FP8MM_X_NOMMA
+            if (!kShared || at.block * Cfg::kStageBlocks + my_block < blocks) {  // a tile's last stage may be half full
 #pragma unroll
-            for (int k = 0; k < kMmasPerBlock; ++k) {
-              // next K=32 slice: 32 bytes further inside the swizzle row (K-major) or 32 rows further
-              umma_f8<PAIR>(d_addr, a_lo + a_kstep * k, b_lo + b_kstep * k, a_hi, b_hi, idesc, k > 0 ? 1u : 0u);
+              for (int k = 0; k < kMmasPerBlock; ++k) {
+                // next K=32 slice: 32 bytes further inside the swizzle row (K-major) or 32 rows further
+                umma_f8<PAIR>(d_addr, a_lo + a_kstep * k, b_lo + b_kstep * k, a_hi, b_hi, idesc, k > 0 ? 1u : 0u);
+              }
             }
-#endif
             umma_commit<PAIR>(smem_u32(&done_bar[at.stage]));
-            at.next(me, p.issuers, stages, nbufs);
+            at.next(kShared ? 0 : me, kShared ? 1 : Cfg::kIssuers, stages, nbufs);
           }
-          at.block -= blocks;
+          at.block -= uses;
         }
       }
       __syncwarp();
@@ -1274,7 +1319,7 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         }
 
 #pragma unroll
-        for (int u = 0; u < kScaleGroup; ++u) {
+        for (int u = 0; u < kScaleGroup; u += Cfg::kStageBlocks) {
           if (kb0 + u >= it.kb_end) break;
           if (!(Cfg::kEarlyProbe && ready_next)) {
             if (!warp_wait(ready_base + static_cast<uint32_t>(cstage * 8), cphase, 0x400 | cstage)) {
@@ -1283,48 +1328,52 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             }
           }
           tcgen05_fence_after();
-          const uint32_t taddr = tmem_base + lane_addr + static_cast<uint32_t>(buf * BN + col_base);
+          const uint32_t taddr = tmem_base + lane_addr + static_cast<uint32_t>(buf * Cfg::kStageBlocks * BN + col_base);
           constexpr int CC = Cfg::kChunkCols;
-          uint32_t v[CC];
-#ifdef FP8MM_X_NOPROMO
-#pragma unroll
-          for (int j = 0; j < CC; ++j) v[j] = 0;
-#else
-          tmem_ld(taddr, v);
-#endif
-#pragma unroll
-          for (int ch = 0; ch < Cfg::kChunks; ++ch) {
-#ifndef FP8MM_X_NOPROMO
-            tmem_ld_wait(v);
-#endif
-            if (ch + 1 == Cfg::kChunks) {
-              // Every column of this buffer is in registers (tcgen05.wait::ld has returned in every
-              // lane once __syncwarp is passed): hand it back to the MMA warp.
-              __syncwarp();
-              release_to(rel_stage);
-              if (++rel_stage == stages) rel_stage = 0;
-              if constexpr (Cfg::kEarlyProbe) {
-                int ns = cstage + 1;
-                uint32_t np = cphase;
-                if (ns == stages) {
-                  ns = 0;
-                  np ^= 1u;
-                }
-                ready_next = mbar_test(ready_base + static_cast<uint32_t>(ns * 8), np);
+          // The buffer has been read: hand it back to the MMA threads, and ask for what comes next.
+          auto drained = [&]() {
+            // Every column of this buffer is in registers (tcgen05.wait::ld has returned in every
+            // lane once __syncwarp is passed).
+            __syncwarp();
+            release_to(rel_stage);
+            if (++rel_stage == stages) rel_stage = 0;
+            if constexpr (Cfg::kEarlyProbe) {
+              int ns = cstage + 1;
+              uint32_t np = cphase;
+              if (ns == stages) {
+                ns = 0;
+                np ^= 1u;
               }
-              // The next group's scales: a non-blocking probe of their slot's barrier, issued here so that its
-              // answer arrives under this K block's fmas. The loader runs slots ahead, so the answer is normally
-              // yes and the blocking wait (a few hundred clocks even on a complete barrier while the
-              // shared-memory path is busy) is skipped.
-              if (u == kScaleGroup - 1) scale_ready = mbar_test(smem_u32(&scale_full_bar[slot]), sphase);
+              ready_next = mbar_test(ready_base + static_cast<uint32_t>(ns * 8), np);
             }
-#ifdef FP8MM_X_NOPROMO
-            if (ch > 0) continue;
-#endif
-            fma_cols(v, ch, s_lo[u], s_hi[u]);
-#ifndef FP8MM_X_NOPROMO
-            if (ch + 1 < Cfg::kChunks) tmem_ld(taddr + static_cast<uint32_t>((ch + 1) * CC), v);
-#endif
+            // The next group's scales: a non-blocking probe of their slot's barrier, issued here so that its
+            // answer arrives under this stage's fmas. The loader runs slots ahead, so the answer is normally
+            // yes and the blocking wait (a few hundred clocks even on a complete barrier while the
+            // shared-memory path is busy) is skipped.
+            if (u + Cfg::kStageBlocks == kScaleGroup) scale_ready = mbar_test(smem_u32(&scale_full_bar[slot]), sphase);
+          };
+          if constexpr (Cfg::kStageBlocks > 1) {
+            // Both K blocks' partials are fetched before the buffer goes back; there is no second one at the end of an odd
+            // range, whose columns are fetched all the same and not used.
+            uint32_t v[Cfg::kStageBlocks][CC];
+#pragma unroll
+            for (int i = 0; i < Cfg::kStageBlocks; ++i) tmem_ld(taddr + static_cast<uint32_t>(i * BN), v[i]);
+#pragma unroll
+            for (int i = 0; i < Cfg::kStageBlocks; ++i) tmem_ld_wait(v[i]);
+            drained();
+#pragma unroll
+            for (int i = 0; i < Cfg::kStageBlocks; ++i)
+              if (i == 0 || kb0 + u + i < it.kb_end) fma_cols(v[i], 0, s_lo[u + i], s_hi[u + i]);
+          } else {
+            uint32_t v[CC];
+            tmem_ld(taddr, v);
+#pragma unroll
+            for (int ch = 0; ch < Cfg::kChunks; ++ch) {
+              tmem_ld_wait(v);
+              if (ch + 1 == Cfg::kChunks) drained();
+              fma_cols(v, ch, s_lo[u], s_hi[u]);
+              if (ch + 1 < Cfg::kChunks) tmem_ld(taddr + static_cast<uint32_t>((ch + 1) * CC), v);
+            }
           }
           if (++buf == nbufs) buf = 0;
           if (++cstage == stages) {
@@ -1420,9 +1469,6 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
         const int sw = (row_in_tile >> 1) & 3;
         constexpr int kBoxes = Cfg::kColsPerThread / kStoreBoxCols;
         auto stage_box = [&](int ch, int bufi) {
-#ifdef FP8MM_X_NOSTAGE
-          return;
-#endif
           uint8_t* rowp = my_stage + bufi * kStoreBufBytes + row_in_tile * 64;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
@@ -1436,9 +1482,6 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
           }
         };
         auto store_box = [&](int ch, int bufi) {
-#ifdef FP8MM_X_NOSTOREISSUE
-          return;
-#endif
           if (MODE == kGrouped) {
             tma_store_3d(&tmap_c, smem_u32(my_stage + bufi * kStoreBufBytes), col0 + ch * kStoreBoxCols,
                          it.m0 + static_cast<int>(cta_rank) * kBlockM, it.group);
@@ -1635,9 +1678,9 @@ EncodeTiledFn get_encode_fn() {
 // costs the host about as much as a small GEMM runs on the device).
 struct MapKey {
   const void* base;
-  cuuint64_t dims[3];
-  cuuint64_t strides[2];
-  cuuint32_t box[3];
+  cuuint64_t dims[4];
+  cuuint64_t strides[3];
+  cuuint32_t box[4];
   int rank;
   int dtype;
   int swizzle;
@@ -1662,12 +1705,11 @@ bool encode_map(CUtensorMap* map, const MapKey& key_in) {
   MapKey key;
   memset(&key, 0, sizeof(key));  // padding bytes take part in the comparison
   key.base = key_in.base;
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < 4; ++i) {
     key.dims[i] = key_in.dims[i];
     key.box[i] = key_in.box[i];
+    if (i < 3) key.strides[i] = key_in.strides[i];
   }
-  key.strides[0] = key_in.strides[0];
-  key.strides[1] = key_in.strides[1];
   key.rank = key_in.rank;
   key.dtype = key_in.dtype;
   key.swizzle = key_in.swizzle;
@@ -1683,7 +1725,7 @@ bool encode_map(CUtensorMap* map, const MapKey& key_in) {
       return true;
     }
   }
-  const cuuint32_t elem_strides[3] = {1, 1, 1};
+  const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
   const CUresult r = fn(map, static_cast<CUtensorMapDataType>(key.dtype), static_cast<cuuint32_t>(key.rank),
                         const_cast<void*>(key.base), key.dims, key.strides, key.box, elem_strides,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, static_cast<CUtensorMapSwizzle>(key.swizzle),
@@ -1699,8 +1741,10 @@ bool encode_map(CUtensorMap* map, const MapKey& key_in) {
 // e4m3 matrix of `rows` rows (M or N) and K columns. K-major (K contiguous, row pitch ld): box = 128 bytes of
 // K x box_rows rows, 128-byte swizzle. MN-major (rows contiguous, ld bytes between consecutive k): box =
 // box_rows (128 or 64) bytes of rows x 128 k, swizzle span = the box's inner extent.
+// `blocks`: K blocks per copy. K-major: K is then two dimensions, the byte of a block and the block, so that a box holds
+// one K block's tile behind the other. MN-major: a box of that many times 128 k.
 bool encode_operand_map(CUtensorMap* map, const void* base, int rows, int K, long long ld, int box_rows,
-                        bool mn_major) {
+                        bool mn_major, int blocks) {
   MapKey k;
   memset(&k, 0, sizeof(k));
   k.base = base;
@@ -1709,7 +1753,14 @@ bool encode_operand_map(CUtensorMap* map, const void* base, int rows, int K, lon
   k.dims[1] = static_cast<cuuint64_t>(mn_major ? K : rows);
   k.strides[0] = static_cast<cuuint64_t>(ld);
   k.box[0] = static_cast<cuuint32_t>(mn_major ? box_rows : kBlockK);
-  k.box[1] = static_cast<cuuint32_t>(mn_major ? kBlockK : box_rows);
+  k.box[1] = static_cast<cuuint32_t>(mn_major ? blocks * kBlockK : box_rows);
+  if (!mn_major && blocks > 1) {
+    k.rank = 3;
+    k.dims[0] = kBlockK;
+    k.dims[2] = static_cast<cuuint64_t>(K / kBlockK);
+    k.strides[1] = kBlockK;
+    k.box[2] = static_cast<cuuint32_t>(blocks);
+  }
   k.dtype = CU_TENSOR_MAP_DATA_TYPE_UINT8;
   k.swizzle = (mn_major && box_rows == 64) ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
   k.l2 = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
@@ -1734,21 +1785,23 @@ bool encode_output_map(CUtensorMap* map, void* base, int M, int N, long long ldc
 }
 
 // Grouped operands: e4m3 [groups][rows][K] with K contiguous, row pitch ld and group pitch lg (bytes);
-// box = 128 bytes of K x box_rows rows of one group.
-bool encode_operand_map_3d(CUtensorMap* map, const void* base, int groups, int rows, int K, long long ld,
-                           long long lg, int box_rows) {
+// box = 128 bytes of K x box_rows rows x `blocks` K blocks of one group.
+bool encode_grouped_operand_map(CUtensorMap* map, const void* base, int groups, int rows, int K, long long ld,
+                                long long lg, int box_rows, int blocks) {
   MapKey k;
   memset(&k, 0, sizeof(k));
   k.base = base;
-  k.rank = 3;
-  k.dims[0] = static_cast<cuuint64_t>(K);
-  k.dims[1] = static_cast<cuuint64_t>(rows);
-  k.dims[2] = static_cast<cuuint64_t>(groups);
-  k.strides[0] = static_cast<cuuint64_t>(ld);
-  k.strides[1] = static_cast<cuuint64_t>(lg);
-  k.box[0] = static_cast<cuuint32_t>(kBlockK);
-  k.box[1] = static_cast<cuuint32_t>(box_rows);
-  k.box[2] = 1;
+  int d = 0;
+  auto dimension = [&](long long extent, long long stride, int box) {
+    k.dims[d] = static_cast<cuuint64_t>(extent);
+    if (d > 0) k.strides[d - 1] = static_cast<cuuint64_t>(stride);
+    k.box[d++] = static_cast<cuuint32_t>(box);
+  };
+  dimension(blocks > 1 ? kBlockK : K, 1, kBlockK);
+  dimension(rows, ld, box_rows);
+  if (blocks > 1) dimension(K / kBlockK, kBlockK, blocks);
+  dimension(groups, lg, 1);
+  k.rank = d;
   k.dtype = CU_TENSOR_MAP_DATA_TYPE_UINT8;
   k.swizzle = CU_TENSOR_MAP_SWIZZLE_128B;
   k.l2 = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
@@ -1809,8 +1862,6 @@ int smem_bytes_for(int block_n, int stages, int pair, int store_bufs) {
 
 constexpr int kMaxSmem = 232448;  // 227 KiB opt-in limit per CTA on sm_100
 
-int tmem_bufs_for(int block_n) { return block_n <= 128 ? 4 : 2; }
-
 // K block j uses ring stage j mod stages and TMEM buffer j mod buffers; the two counts are independent
 // (the promotion warps release a buffer to the barrier of the stage that the K block `buffers` later will
 // use), except that a buffer cannot be re-used before its stage is: buffers <= stages.
@@ -1819,8 +1870,8 @@ int tmem_bufs_in_use(int block_n, int stages) {
   return d < stages ? d : stages;
 }
 
-// MMA-issuing threads (see the kernel).
-int issuers_for(int block_n) { return block_n <= 128 ? 2 : 1; }
+// A plan counts its ring in K blocks; where a stage has two, an odd last one is left unused.
+int ring_stages(const b200_fp8_mm_plan& pl) { return pl.stages / stage_blocks_for(pl.block_n); }
 
 // Deepest ring that fits. The 256-wide tiles stop at four stages: a fifth measured 5 % slower (their
 // promotion warps still spill a little, and local memory loses L1 to every extra stage). Where two issuers share the
@@ -1909,7 +1960,7 @@ bool runs_as_cluster(const b200_fp8_mm_plan& pl, int sm_count) {
   if (pl.cta_pair || pl.full_tiles != 0 || pl.split_k < 2 || pl.split_k > kMaxCluster) return false;
   if (pl.block_n != 64 && pl.block_n != 128) return false;
   if (pl.tiles > cluster_capacity(pl.split_k, sm_count)) return false;
-  return pl.stages * (kBlockM + pl.block_n) * kBlockK >= kBlockM * (pl.block_n + 4) * 4;
+  return ring_stages(pl) * stage_blocks_for(pl.block_n) * (kBlockM + pl.block_n) * kBlockK >= kBlockM * (pl.block_n + 4) * 4;
 }
 
 // Cost of a split plan that runs as clusters, in the selector's clocks, fitted to timings of every such plan over 28
@@ -2245,8 +2296,9 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   const OperandLayout la = operand_layout(a_mn, kBlockM);
   const OperandLayout lb = operand_layout(b_mn, b_box_rows_for(pl.block_n, pl.cta_pair));
   const int a_box = a_mn ? la.box_cols : a_box_rows_for(M);
-  if (!encode_operand_map(&map_a, a, M, K, lda, a_box, a_mn)) return B200_FP8_MM_ERR_DRIVER;
-  if (!encode_operand_map(&map_b, b, N, K, ldb, lb.box_cols, b_mn)) return B200_FP8_MM_ERR_DRIVER;
+  const int blocks = stage_blocks_for(pl.block_n);
+  if (!encode_operand_map(&map_a, a, M, K, lda, a_box, a_mn, blocks)) return B200_FP8_MM_ERR_DRIVER;
+  if (!encode_operand_map(&map_b, b, N, K, ldb, lb.box_cols, b_mn, blocks)) return B200_FP8_MM_ERR_DRIVER;
 
   KernelParams kp;
   memset(&kp, 0, sizeof(kp));
@@ -2270,9 +2322,12 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   kp.split_k = pl.split_k;
   kp.full_tiles = pl.full_tiles;
   kp.kblocks = kblocks;
-  kp.stages = pl.stages;
-  kp.stage_tx = static_cast<uint32_t>((a_box + b_box_rows_for(pl.block_n, pl.cta_pair)) * kBlockK);
-  kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
+  kp.stages = ring_stages(pl);
+  // (an MN-major a comes in boxes of 128 rows, whatever M is)
+  const int a_rows = a_mn ? kBlockM : a_box;
+  kp.stage_tx = static_cast<uint32_t>(blocks * (a_rows + b_box_rows_for(pl.block_n, pl.cta_pair)) * kBlockK);
+  kp.a_block_bytes = static_cast<uint32_t>(a_rows * kBlockK);
+  kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, kp.stages);
   kp.store_bufs = store_bufs;
   kp.a_mn = a_mn ? 1 : 0;
   kp.b_mn = b_mn ? 1 : 0;
@@ -2286,9 +2341,6 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   kp.b_desc_hi = lb.desc_hi;
   kp.b_kstep = lb.kstep;
   kp.idesc_major = (a_mn ? (1u << 15) : 0u) | (b_mn ? (1u << 16) : 0u);
-  // Two issuing threads pay off where the MMAs are short (narrow tiles: 25 % faster at block_n 64,
-  // 10 % at 128); the wide tiles are bound by the promotion warps and run 1 % better with one.
-  kp.issuers = issuers_for(pl.block_n);
   {
     // Tile rows per raster group: the tiles running at one time form a block as square as possible.
     const int units = pl.cta_pair ? sm_count / 2 : sm_count;
@@ -2338,7 +2390,9 @@ int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUte
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(static_cast<unsigned>(pl.grid), 1, 1);
   cfg.blockDim = dim3(static_cast<unsigned>(128 + 32 * epi_warps_for(pl.block_n)), 1, 1);
-  cfg.dynamicSmemBytes = static_cast<size_t>(pl.smem_bytes);
+  // Never less than half of an SM's shared memory, so that no two CTAs of a launch share an SM: a second would wait for the
+  // first's TMEM, and two pairs or clusters placed across the same two SMs could wait for each other.
+  cfg.dynamicSmemBytes = static_cast<size_t>(pl.smem_bytes > kMaxSmem / 2 ? pl.smem_bytes : kMaxSmem / 2 + 1024);
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see pdl_wait() in the kernel
@@ -2415,9 +2469,10 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
     memset(&map_c, 0, sizeof(map_c));
   }
   const int a_box = a_box_rows_for(M);
-  if (!encode_operand_map_3d(&map_a, a, groups, M, K, lda, a_g, a_box)) return B200_FP8_MM_ERR_DRIVER;
+  const int blocks = stage_blocks_for(pl.block_n);
+  if (!encode_grouped_operand_map(&map_a, a, groups, M, K, lda, a_g, a_box, blocks)) return B200_FP8_MM_ERR_DRIVER;
   const int b_rows_per_cta = b_box_rows_for(pl.block_n, pl.cta_pair);
-  if (!encode_operand_map_3d(&map_b, b, groups, N, K, ldb, b_g, b_rows_per_cta)) return B200_FP8_MM_ERR_DRIVER;
+  if (!encode_grouped_operand_map(&map_b, b, groups, N, K, ldb, b_g, b_rows_per_cta, blocks)) return B200_FP8_MM_ERR_DRIVER;
 
   const OperandLayout la = operand_layout(false, kBlockM);
   const OperandLayout lb = operand_layout(false, b_rows_per_cta);
@@ -2440,9 +2495,10 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.split_k = 1;
   kp.full_tiles = groups * kp.tiles_m * kp.tiles_n;
   kp.kblocks = K / kBlockK;
-  kp.stages = pl.stages;
-  kp.stage_tx = static_cast<uint32_t>((a_box + b_rows_per_cta) * kBlockK);
-  kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, pl.stages);
+  kp.stages = ring_stages(pl);
+  kp.stage_tx = static_cast<uint32_t>(blocks * (a_box + b_rows_per_cta) * kBlockK);
+  kp.a_block_bytes = static_cast<uint32_t>(a_box * kBlockK);
+  kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, kp.stages);
   kp.store_bufs = store_bufs;
   kp.b_boxes = lb.boxes;
   kp.b_box_cols = lb.box_cols;
@@ -2453,7 +2509,6 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.b_desc_lo = lb.desc_lo;
   kp.b_desc_hi = lb.desc_hi;
   kp.b_kstep = lb.kstep;
-  kp.issuers = issuers_for(pl.block_n);
   {
     const int units = pl.cta_pair ? sm_count / 2 : sm_count;
     int g = (units + kp.tiles_n / 2) / kp.tiles_n;
