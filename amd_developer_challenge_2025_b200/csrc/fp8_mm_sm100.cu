@@ -1983,6 +1983,14 @@ Candidate evaluate(int M, int N, int kblocks, int sm_count, int bn, int pair, in
   return best;
 }
 
+// 128-wide single CTAs with one tile each: nothing runs under the TMA store of a tile, so its rows leave straight from registers
+// (store_row), and without the second staging buffer the ring has six stages for four, which pays from about as many K blocks on
+// (2048 x 512 x 7168 24.1 -> 20.1 us, 369 x 3196 x 1792 10.1 -> 9.0, 1500 x 1000 x 2048 10.4 -> 9.9). With several tiles a CTA
+// the TMA store is ahead (2048 x 7168 x 512 19.1 against 20.9).
+bool long_ring(int bn, int pair, int split, int tiles, int units, int kblocks) {
+  return bn == 128 && !pair && split == 1 && tiles <= units && kblocks > 6;
+}
+
 // The launch plan of a candidate.
 void fill_plan(int M, int N, int kblocks, int sm_count, const b200_fp8_mm_plan* forced, const Candidate& best,
                b200_fp8_mm_plan* out) {
@@ -1995,6 +2003,8 @@ void fill_plan(int M, int N, int kblocks, int sm_count, const b200_fp8_mm_plan* 
   if (store_bufs < 0)
     store_bufs = (full_tiles == 0 || !valid_block_n(bn)) ? 0 : store_bufs_for(bn, pair, kblocks);
   if (full_tiles == 0 && best.split > 1) store_bufs = 0;  // every tile leaves through the fp32 planes first
+  if ((forced == nullptr || (forced->store_bufs == 0 && forced->stages == 0)) && long_ring(bn, pair, best.split, tiles, units, kblocks))
+    store_bufs = 1;
   const int stages =
       (forced && forced->stages) ? forced->stages : (valid_block_n(bn) ? max_stages_for(bn, pair, store_bufs) : 2);
   out->block_m = kBlockM;
@@ -2029,12 +2039,12 @@ double choose_plan(int M, int N, int K, int sm_count, const b200_fp8_mm_plan* fo
     }
   }
   if (best.bn == 0) best = Candidate{f_bn, f_pair > 0 ? 1 : 0, 1, 0, 0.0};  // invalid forced width
-  // 64-wide pairs halve what a CTA loads of b per K block but take longer to start and to finish: below about 20 K blocks
-  // single CTAs are faster (1024 x 1024 x 1024 5.7 against 6.5 us, 300 x 2000 x 512 4.7 against 5.6, 129 x 4099 x 2304 10.7
-  // against 11.5), from there on they are not (200 x 2000 x 2560 8.5 against 8.4, 900 x 256 x 6144 15.1 against 14.7).
-  // (They stay ahead of the wider tiles that the pair was ahead of: 909 x 2325 x 1152 13.5 us, 192-wide pairs 16.8. From here on
-  // the cost is the single-CTA plan's own, so that it is what clusters have to beat: 945 x 541 x 2304 10.1 us, two ranges 8.3.)
-  if (f_pair < 0 && best.pair && best.bn == 64 && best.split == 1 && kblocks < 20)
+  // 64-wide pairs halve what a CTA loads of b per K block but take longer to start, to finish and to hand a K block over: single
+  // CTAs are faster (two K blocks a stage: 2048 x 576 x 7168 15.8 against 16.5 us, 512 x 1536 x 7168 15.0 against 15.9,
+  // 1024 x 1024 x 1024 5.6 against 6.4, 129 x 4099 x 2304 8.7 against 9.3).
+  // (They stay ahead of the wider tiles that the pair was ahead of: 909 x 2325 x 1152 10.0 us, 192-wide pairs 11.2. From here on
+  // the cost is the single-CTA plan's own, so that it is what clusters have to beat.)
+  if (f_pair < 0 && best.pair && best.bn == 64 && best.split == 1)
     best = evaluate(M, N, kblocks, sm_count, best.bn, 0, 1);
   fill_plan(M, N, kblocks, sm_count, forced, best, out);
   // What the caller's workspace must hold is decided by this plan. Running the ranges as clusters needs none, so a
@@ -2252,6 +2262,7 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
 
   CUtensorMap map_a, map_b, map_c;
   int store_bufs = tma_store_fits(c, N, ldc, 0) ? pl.store_bufs : 0;
+  if (forced_in == nullptr && long_ring(pl.block_n, pl.cta_pair, pl.split_k, pl.tiles, sm_count, kblocks)) store_bufs = 0;
   if (store_bufs > 0) {
     if (!encode_output_map(&map_c, c, M, N, ldc)) return B200_FP8_MM_ERR_DRIVER;
   } else {
