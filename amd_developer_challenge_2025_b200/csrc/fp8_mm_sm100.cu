@@ -48,6 +48,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <limits.h>
+#include <math.h>
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
@@ -2389,8 +2390,26 @@ int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUte
   return B200_FP8_MM_OK;
 }
 
+// Cost of a grouped launch with row counts, which are device memory and unknown here: rated over loads from 1/8 to all of M,
+// and, at half the weight, with every group full. What a tile of a grouped kernel costs beside its K blocks is more than
+// in the plain kernels, most of all for pairs. (graph, us, tile shape chosen for full groups / this way: 8 x 1024 x 2048 x 7168
+// with loads of 1/8 .. 8/8 98 / 76, 16 x 300 x 1024 x 2048 24.9 / 18.8, 10 x 500 x 3520 x 384 21.2 / 17.1; every group full
+// 128 / 138, half full 70 / 75.)
+double uneven_cost(int groups, int M, int N, int kblocks, int sm_count, int bn, int pair) {
+  const int tile_m = pair ? 2 * kBlockM : kBlockM, units = pair ? sm_count / 2 : sm_count;
+  const WidthCost wc = width_cost(bn, pair);
+  const double extra = pair ? 2000.0 : (bn == 256 ? 500.0 : (bn == 192 ? 1500.0 : 0.0));
+  long long eighths = 0;  // tile rows of eight groups, one of each load
+  for (int i = 1; i <= 8; ++i) eighths += ceil_div(ceil_div(M, 8) * i < M ? ceil_div(M, 8) * i : M, tile_m);
+  auto waves = [&](double tile_rows) { return ceil(tile_rows * ceil_div(N, bn) / units - 1e-9); };
+  const double uneven = waves(ceil(static_cast<double>(groups) * static_cast<double>(eighths) / 8.0));
+  const double full = waves(static_cast<double>(groups) * ceil_div(M, tile_m));
+  return (uneven + 0.5 * full) * (kblocks * wc.per_kblock + wc.per_tile + extra);
+}
+
 // Grouped launch: `groups` problems of the same N and K in one kernel. Every tile is a whole tile (no split-K); its shape
-// is chosen as for one GEMM with all groups' row blocks stacked, CTA pairs only where a group's rows fill their tiles.
+// is chosen as for one GEMM with all groups' row blocks stacked, CTA pairs only where a group's rows fill their tiles; with row
+// counts by uneven_cost().
 int run_grouped(const void* a, const void* b, const float* a_scale, const float* b_scale, void* c, int groups, int M,
                 int N, int K, long long lda, long long a_g, long long ldb, long long b_g, long long sa_g,
                 long long sa_m, long long sa_k, long long sb_g, long long sb_n, long long sb_k, long long ldc,
@@ -2430,6 +2449,22 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   if (!pl.cta_pair || forced.cta_pair < 0) {
     forced.cta_pair = -1;
     choose_plan(groups * ceil_div(M, kBlockM) * kBlockM, N, K, sm_count, &forced, &pl);
+  }
+  if (m_valid != nullptr && forced_in == nullptr) {
+    double best = 1e300;
+    b200_fp8_mm_plan shape;
+    memset(&shape, 0, sizeof(shape));
+    shape.split_k = 1;
+    for (int pair = pair_fits ? 1 : 0; pair >= 0; --pair) {
+      for (int bn = 256; bn >= (pair ? 192 : 64); bn -= 64) {
+        const double cost = uneven_cost(groups, M, N, K / kBlockK, sm_count, bn, pair);
+        if (cost >= best) continue;
+        best = cost;
+        shape.block_n = bn;
+        shape.cta_pair = pair ? 1 : -1;
+      }
+    }
+    choose_plan(groups * (shape.cta_pair > 0 ? rows256 : ceil_div(M, kBlockM) * kBlockM), N, K, sm_count, &shape, &pl);
   }
   if (!plan_is_supported(pl, K / kBlockK) || pl.split_k != 1) return B200_FP8_MM_ERR_PLAN;
   const int tiles_m = ceil_div(M, pl.cta_pair ? 2 * kBlockM : kBlockM);
