@@ -2683,6 +2683,90 @@ int b200_fp8_mm_grouped(const void* a, const void* b, const float* a_scale, cons
                      sb_k, ldc, c_g, m_valid, device_status, stream, forced);
 }
 
+int b200_fp8_mm_host_ranges(const void* a, const void* b, const float* a_scale, const float* b_scale, void* c, int M, int N,
+                            int K, int n_phase, int by_columns, const int* cuts, int ranges, void* d_a, void* d_b,
+                            float* d_a_scale, float* d_b_scale, void* d_c, void* workspace, size_t workspace_bytes,
+                            int* device_status, void* caller_stream, void* in_stream, void* mm_stream, void* out_stream) {
+  if (a == nullptr || b == nullptr || a_scale == nullptr || b_scale == nullptr || c == nullptr || d_a == nullptr ||
+      d_b == nullptr || d_a_scale == nullptr || d_b_scale == nullptr || d_c == nullptr || cuts == nullptr)
+    return B200_FP8_MM_ERR_NULL;
+  const int extent = by_columns ? N : M;
+  if (M <= 0 || N <= 0 || K <= 0 || (K % kBlockK) != 0 || ranges < 1 || cuts[0] != 0 || cuts[ranges] != extent)
+    return B200_FP8_MM_ERR_SHAPE;
+  for (int i = 0; i < ranges; ++i)
+    if (cuts[i] >= cuts[i + 1] || (by_columns && cuts[i] % kBlockK != 0)) return B200_FP8_MM_ERR_SHAPE;
+  if (n_phase < 0 || n_phase >= 128 || (n_phase % 32) != 0) return B200_FP8_MM_ERR_PHASE;
+  const size_t m = M, n = N, k = K, kb = k / kBlockK, nb = (n + n_phase + 127) / 128;
+  cudaStream_t in = static_cast<cudaStream_t>(in_stream);
+  // One range has nothing to overlap: all on one stream, no events.
+  cudaStream_t mm = ranges > 1 ? static_cast<cudaStream_t>(mm_stream) : in;
+  cudaStream_t out = ranges > 1 ? static_cast<cudaStream_t>(out_stream) : in;
+  int rc = B200_FP8_MM_OK;
+  auto call = [&](cudaError_t err) {
+    if (err == cudaSuccess) return;
+    (void)cudaGetLastError();
+    if (rc == B200_FP8_MM_OK) rc = B200_FP8_MM_ERR_LAUNCH;
+  };
+  cudaEvent_t event = nullptr;
+  call(cudaEventCreateWithFlags(&event, cudaEventDisableTiming));
+  if (rc != B200_FP8_MM_OK) return rc;
+  // (one event serves every hand-over: a wait takes the record that is the latest when the wait is issued)
+  auto after = [&](cudaStream_t next, cudaStream_t first) {
+    if (next == first) return;
+    call(cudaEventRecord(event, first));
+    call(cudaStreamWaitEvent(next, event, 0));
+  };
+  auto to_device = [&](void* dst, const void* src, size_t bytes) {
+    call(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, in));
+  };
+  const char* h_a = static_cast<const char*>(a);
+  const char* h_b = static_cast<const char*>(b);
+  char* h_c = static_cast<char*>(c);
+  char* g_a = static_cast<char*>(d_a);
+  char* g_b = static_cast<char*>(d_b);
+  char* g_c = static_cast<char*>(d_c);
+  // whatever the caller's stream still has to do comes first
+  after(in, static_cast<cudaStream_t>(caller_stream));
+  if (by_columns) {
+    to_device(g_a, h_a, m * k);
+  } else {
+    to_device(g_b, h_b, n * k);
+  }
+  to_device(d_a_scale, a_scale, m * kb * sizeof(float));
+  to_device(d_b_scale, b_scale, nb * kb * sizeof(float));
+  for (int i = 0; i < ranges && rc == B200_FP8_MM_OK; ++i) {
+    const size_t r0 = cuts[i], rows = cuts[i + 1] - r0;
+    if (by_columns) {
+      to_device(g_b + r0 * k, h_b + r0 * k, rows * k);
+    } else {
+      to_device(g_a + r0 * k, h_a + r0 * k, rows * k);
+    }
+    after(mm, in);
+    if (rc != B200_FP8_MM_OK) break;
+    if (by_columns) {  // a block of columns has a piece of d_c of its own, rows of `rows` elements
+      rc = run(g_a, g_b + r0 * k, d_a_scale, d_b_scale + r0 / 128 * kb, g_c + 2 * m * r0, M, static_cast<int>(rows), K, K, 1, K, 1,
+               kb, 1, kb, 1, static_cast<long long>(rows), n_phase, workspace, workspace_bytes, device_status, mm, nullptr);
+    } else {
+      rc = run(g_a + r0 * k, g_b, d_a_scale + r0 * kb, d_b_scale, g_c + 2 * n * r0, static_cast<int>(rows), N, K, K, 1, K, 1, kb,
+               1, kb, 1, N, n_phase, workspace, workspace_bytes, device_status, mm, nullptr);
+    }
+    if (rc != B200_FP8_MM_OK) break;
+    after(out, mm);
+    if (by_columns && rows != n) {
+      call(cudaMemcpy2DAsync(h_c + 2 * r0, 2 * n, g_c + 2 * m * r0, 2 * rows, 2 * rows, m, cudaMemcpyDeviceToHost, out));
+    } else {
+      const size_t first = by_columns ? 0 : 2 * n * r0;
+      call(cudaMemcpyAsync(h_c + first, g_c + first, by_columns ? 2 * m * n : 2 * n * rows, cudaMemcpyDeviceToHost, out));
+    }
+  }
+  // (waited for after a failure too: the caller's buffers may not be in use when this returns)
+  call(cudaStreamSynchronize(in));
+  if (mm != in) call(cudaStreamSynchronize(mm));
+  if (out != in) call(cudaStreamSynchronize(out));
+  (void)cudaEventDestroy(event);
+  return rc;
+}
+
 size_t b200_fp8_mm_static_scratch_limit(void) { return kStaticScratchBytes; }
 
 size_t b200_fp8_mm_workspace_bytes(int M, int N, int K) {

@@ -5,6 +5,7 @@ Mirrors the reference's pybind launcher `fp8_mm(a, b, as, bs, c, c_tmp)`
 from __future__ import annotations
 
 import ctypes
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -297,6 +298,7 @@ class _HostPipeline:
         self.s_in = torch.cuda.Stream(dev)
         self.s_mm = torch.cuda.Stream(dev)
         self.s_out = torch.cuda.Stream(dev)
+        self.lock = threading.Lock()  # the buffers serve one call at a time
         self.key = None
         self.bufs = None
 
@@ -337,13 +339,42 @@ def host_row_chunks(m: int, chunk_rows: int = 1024) -> list[tuple[int, int]]:
     return out
 
 
+# Bytes in and out from which a problem is cut into ranges (below, events and further copies cost more than they hide: 4.3 MB in
+# one 148 us, in two 138; 0.4 MB 81 and 78), and from which it gets one more (7.8 MB in two or three 204 us, in six 214; 35 MB in
+# four 649, in two 670; 67 MB in six 1075, in three 1095, in one 1330).
+HOST_RANGE_BYTES = 3 << 20
+HOST_FURTHER_RANGE_BYTES = 16 << 20
+
+
+def host_ranges(m: int, n: int, k: int, chunk_rows: int = 1024) -> tuple[bool, list[int]]:
+    """How the host entry point cuts a problem: whether b (else a) is the operand that arrives in ranges, and the cuts.
+
+    Nothing can travel back before one operand is there in full: that is the smaller one (1112 x 4305 x 2816 by columns 455 us, by
+    rows 497; 300 x 4608 x 1024 203 and 216), and the larger one arrives in equal ranges of at most `chunk_rows` rows (of b: columns
+    of c), or with short ranges at both ends where there are many."""
+    by_columns = n > m and chunk_rows > 0 and chunk_rows % SCALE_BLOCK == 0
+    extent = n if by_columns else m
+    moved = m * k + n * k + 2 * m * n
+    if moved < HOST_RANGE_BYTES or extent <= 2 * SCALE_BLOCK:
+        return by_columns, [0, extent]
+    if extent > 4 * chunk_rows:
+        inner = [r1 for _, r1 in host_row_chunks(extent, chunk_rows)[:-1]]
+    else:
+        parts = max(2 + moved // HOST_FURTHER_RANGE_BYTES, -(-extent // chunk_rows))
+        rows = -(-extent // (parts * SCALE_BLOCK)) * SCALE_BLOCK
+        inner = list(range(rows, extent, rows))
+    if by_columns:
+        inner = [r // SCALE_BLOCK * SCALE_BLOCK for r in inner]
+    return by_columns, [0] + inner + [extent]
+
+
 def fp8_mm_host(a, b, a_scale, b_scale, c, device="cuda", n_phase: int = 0, chunk_rows: int = 1024):
     """The same operator for HOST tensors (pinned memory for full speed): returns c, filled, when done.
 
-    b, b_scale and a_scale are copied to `device` first; a is then streamed in row ranges, each range's
-    GEMM runs as soon as its rows have landed, and its rows of c are copied back while later ranges are
-    still arriving, so both directions of the host link and the SMs work at the same time (three
-    streams, events between them). Every range is an independent GEMM over whole rows with the plan the
+    The smaller operand and the scales are copied to `device` first; the larger one is then streamed in row ranges
+    (`host_ranges`), each range's GEMM runs as soon as its rows have landed, and its part of c is copied back while later
+    ranges are still arriving, so both directions of the host link and the SMs work at the same time (three
+    streams, events between them). Every range is an independent GEMM with the plan the
     library picks for its size; the result meets the same tolerance as one GEMM over the whole problem
     (and equals it bit for bit unless a range's plan splits K, which only changes the order in which K
     ranges are added). Device buffers are kept per device between calls of the same shape. This is the
@@ -360,6 +391,51 @@ def fp8_mm_host(a, b, a_scale, b_scale, c, device="cuda", n_phase: int = 0, chun
     pipe = _host_pipelines.get(dev.index)
     if pipe is None:
         pipe = _host_pipelines[dev.index] = _HostPipeline(dev)
+    with pipe.lock:
+        if _plain_host_call(a, b, a_scale, b_scale, c, n_phase):
+            _host_call(pipe, a, b, a_scale, b_scale, c, n_phase, chunk_rows)
+        else:
+            _host_call_converting(pipe, a, b, a_scale, b_scale, c, n_phase, chunk_rows)
+    return c
+
+
+def _plain_host_call(a, b, a_scale, b_scale, c, n_phase) -> bool:
+    """Whether the bytes can be copied as they are: the operator's own types and shapes."""
+    if not (isinstance(n_phase, int) and a.dtype == b.dtype == torch.float8_e4m3fn and a_scale.dtype == b_scale.dtype == torch.float32
+            and c.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2 and n_phase in (0, 32, 64, 96)
+            and all(type(t) is torch.Tensor and t.device.type == "cpu" for t in (a, b, a_scale, b_scale, c))):
+        return False
+    m, k = a.shape
+    n = b.shape[0]
+    return (m > 0 and n > 0 and k > 0 and k % SCALE_BLOCK == 0 and b.shape[1] == k and tuple(c.shape) == (m, n)
+            and tuple(a_scale.shape) == (m, k // SCALE_BLOCK)
+            and tuple(b_scale.shape) == ((n + n_phase + SCALE_BLOCK - 1) // SCALE_BLOCK, k // SCALE_BLOCK))
+
+
+def _host_call(pipe, a, b, a_scale, b_scale, c, n_phase, chunk_rows):
+    """The whole pipeline in one library call. Its copies, events and launches took some 100 us of a small problem's 130 to 270
+    one by one from Python."""
+    dev, (m, k), n = pipe.dev, a.shape, b.shape[0]
+    by_columns, cuts = host_ranges(m, n, k, chunk_rows)
+    sizes = {r1 - r0 for r0, r1 in zip(cuts, cuts[1:])}
+    with torch.cuda.device(dev):
+        nbytes = max(workspace_bytes(m, r, k) if by_columns else workspace_bytes(r, n, k) for r in sizes)
+        da, db, das, dbs, dc = pipe.buffers(m, n, k, b_scale.shape[0])
+        ws = _workspace(dev, nbytes, pipe.s_mm.cuda_stream)
+        rc = _lib.load().b200_fp8_mm_host_ranges(
+            a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), c.data_ptr(), m, n, k, n_phase,
+            int(by_columns), (ctypes.c_int * len(cuts))(*cuts), len(cuts) - 1,
+            da.data_ptr(), db.data_ptr(), das.data_ptr(), dbs.data_ptr(), dc.data_ptr(),
+            ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0,
+            _status_words(dev).data_ptr(), torch.cuda.current_stream(dev).cuda_stream,
+            pipe.s_in.cuda_stream, pipe.s_mm.cuda_stream, pipe.s_out.cuda_stream)
+    if rc != 0:
+        raise Fp8MmError(rc, f"M={m} N={n} K={k}")
+
+
+def _host_call_converting(pipe, a, b, a_scale, b_scale, c, n_phase, chunk_rows):
+    """Other types are converted by the copies, and whatever the operator refuses is refused by its own checks."""
+    dev, (m, k), n = pipe.dev, a.shape, b.shape[0]
     da, db, das, dbs, dc = pipe.buffers(m, n, k, b_scale.shape[0])
     caller = torch.cuda.current_stream(dev)
     pipe.s_in.wait_stream(caller)
@@ -381,4 +457,3 @@ def fp8_mm_host(a, b, a_scale, b_scale, c, device="cuda", n_phase: int = 0, chun
                 c[r0:r1].copy_(dc[r0:r1], non_blocking=True)
     pipe.s_out.synchronize()
     caller.wait_stream(pipe.s_out)
-    return c

@@ -243,6 +243,20 @@ int b200_fp8_mm_selftest_wait_expiry(const void* a, const void* b, const float* 
                                      unsigned long long wait_limit_ns, int skip_kblock,
                                      int* device_status, void* stream);
 
+/*
+ * The GEMM for operands and result in host memory (pinned for full speed), contiguous: a [M,K], b [N,K], scales [M,K/128]
+ * and [ceil((N+n_phase)/128),K/128], c [M,N]. One operand is copied to the device first; the other follows in `ranges` ranges of
+ * rows, [cuts[i], cuts[i+1]) with cuts[0] = 0: rows of a, or with `by_columns` rows of b (columns of c), cut at multiples of 128.
+ * Each range's GEMM runs when its rows have landed, and its part of c travels back while later ranges arrive.
+ * d_*: device buffers of the same sizes; workspace as large as any range asks for. Work on caller_stream comes before all of it.
+ * Uses the three other streams and returns when c is complete. (No counterpart in the reference, whose operator takes device
+ * tensors only.)
+ */
+int b200_fp8_mm_host_ranges(const void* a, const void* b, const float* a_scale, const float* b_scale, void* c, int M, int N,
+                            int K, int n_phase, int by_columns, const int* cuts, int ranges, void* d_a, void* d_b,
+                            float* d_a_scale, float* d_b_scale, void* d_c, void* workspace, size_t workspace_bytes,
+                            int* device_status, void* caller_stream, void* in_stream, void* mm_stream, void* out_stream);
+
 /* Size in bytes of the scratch array b200_fp8_mm_static_scratch uses. */
 size_t b200_fp8_mm_static_scratch_limit(void);
 
