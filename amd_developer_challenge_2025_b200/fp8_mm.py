@@ -351,13 +351,13 @@ def host_ranges(m: int, n: int, k: int, chunk_rows: int = 1024) -> tuple[bool, l
 
     Nothing can travel back before one operand is there in full: that is the smaller one (1112 x 4305 x 2816 by columns 455 us, by
     rows 497; 300 x 4608 x 1024 203 and 216), and the larger one arrives in equal ranges of at most `chunk_rows` rows (of b: columns
-    of c), or with short ranges at both ends where there are many."""
+    of c), or with short ranges at both ends where there are many large ones."""
     by_columns = n > m and chunk_rows > 0 and chunk_rows % SCALE_BLOCK == 0
     extent = n if by_columns else m
     moved = m * k + n * k + 2 * m * n
     if moved < HOST_RANGE_BYTES or extent <= 2 * SCALE_BLOCK:
         return by_columns, [0, extent]
-    if extent > 4 * chunk_rows:
+    if extent > 4 * chunk_rows and moved >= 3 * HOST_FURTHER_RANGE_BYTES:
         inner = [r1 for _, r1 in host_row_chunks(extent, chunk_rows)[:-1]]
     else:
         parts = max(2 + moved // HOST_FURTHER_RANGE_BYTES, -(-extent // chunk_rows))
