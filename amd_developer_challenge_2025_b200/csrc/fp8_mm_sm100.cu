@@ -107,7 +107,8 @@ struct KernelParams {
   float rcp_per_group, rcp_raster, rcp_raster_last, rcp_split, rcp_per_problem, rcp_tiles_n;
   int b_scale_rows;
   int stages;              // of TileCfg::kStageBlocks K blocks each
-  uint32_t stage_tx;       // bytes the copies of one stage bring to this CTA
+  int box_blocks;          // K blocks that one copy of an operand brings: all of a stage's, or 1
+  uint32_t copy_tx;        // bytes that one copy of each operand brings to this CTA
   uint32_t a_block_bytes;  // from one K block of a stage's a to the next
   int tmem_bufs;  // TMEM partial buffers in use, each for a stage's K blocks: at most stages and TileCfg::kTmemBufs
   int store_bufs;  // staging buffers per promotion warpgroup for the TMA store of c: 0 (plain stores), 1 .. 4
@@ -1047,39 +1048,47 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             }
             // Both CTAs of a pair report to the leader's barrier: its MMA threads consume the stage.
             const uint32_t fb = PAIR ? map_to_cta(smem_u32(&full_bar[stage]), 0) : smem_u32(&full_bar[stage]);
-            mbar_expect_tx_cluster(fb, p.stage_tx);
+            const int here = min(Cfg::kStageBlocks, it.kb_end - kb);  // K blocks of this stage
+            const int copies = Cfg::kStageBlocks == 1 || p.box_blocks > 1 ? 1 : here;
+            mbar_expect_tx_cluster(fb, static_cast<uint32_t>(copies) * p.copy_tx);
             const uint32_t sa = smem_u32(ring + stage * Cfg::kStageBytes);
             const uint32_t sb = sa + Cfg::kStageBytesA;
             // K-major: x = byte of K, y = matrix row; where a stage has several K blocks, x = byte of a block, y = row,
             // z = block. MN-major: x = matrix row (a multiple of 64), y = k. K blocks past the end of K arrive as zeros.
-            if constexpr (MODE == kGrouped) {
-              if constexpr (Cfg::kStageBlocks > 1) {
-                tma_load_4d<PAIR>(sa, &tmap_a, 0, a_row, kb, it.group, fb);
-                tma_load_4d<PAIR>(sb, &tmap_b, 0, b_row, kb, it.group, fb);
-              } else {
-                tma_load_3d<PAIR>(sa, &tmap_a, kb * kBlockK, a_row, it.group, fb);
-                tma_load_3d<PAIR>(sb, &tmap_b, kb * kBlockK, b_row, it.group, fb);
-              }
-            } else {
-              auto load_k_major = [&](uint32_t dst, const CUtensorMap* map, int row) {
+            auto copy = [&](uint32_t sa, uint32_t sb, int kb) {
+              if constexpr (MODE == kGrouped) {
                 if constexpr (Cfg::kStageBlocks > 1) {
-                  tma_load_3d<PAIR>(dst, map, 0, row, kb, fb);
+                  tma_load_4d<PAIR>(sa, &tmap_a, 0, a_row, kb, it.group, fb);
+                  tma_load_4d<PAIR>(sb, &tmap_b, 0, b_row, kb, it.group, fb);
                 } else {
-                  tma_load_2d<PAIR>(dst, map, kb * kBlockK, row, fb);
+                  tma_load_3d<PAIR>(sa, &tmap_a, kb * kBlockK, a_row, it.group, fb);
+                  tma_load_3d<PAIR>(sb, &tmap_b, kb * kBlockK, b_row, it.group, fb);
                 }
-              };
-              if (MODE != kMnMajor || !p.a_mn) {
-                load_k_major(sa, &tmap_a, a_row);
               } else {
-                tma_load_2d<PAIR>(sa, &tmap_a, a_row, kb * kBlockK, fb);
+                auto load_k_major = [&](uint32_t dst, const CUtensorMap* map, int row) {
+                  if constexpr (Cfg::kStageBlocks > 1) {
+                    tma_load_3d<PAIR>(dst, map, 0, row, kb, fb);
+                  } else {
+                    tma_load_2d<PAIR>(dst, map, kb * kBlockK, row, fb);
+                  }
+                };
+                if (MODE != kMnMajor || !p.a_mn) {
+                  load_k_major(sa, &tmap_a, a_row);
+                } else {
+                  tma_load_2d<PAIR>(sa, &tmap_a, a_row, kb * kBlockK, fb);
+                }
+                if (MODE != kMnMajor || !p.b_mn) {
+                  load_k_major(sb, &tmap_b, b_row);
+                } else {
+                  for (int i = 0; i < p.b_boxes; ++i)
+                    tma_load_2d<PAIR>(sb + static_cast<uint32_t>(i * p.b_box_bytes), &tmap_b, b_row + i * p.b_box_cols,
+                                      kb * kBlockK, fb);
+                }
               }
-              if (MODE != kMnMajor || !p.b_mn) {
-                load_k_major(sb, &tmap_b, b_row);
-              } else {
-                for (int i = 0; i < p.b_boxes; ++i)
-                  tma_load_2d<PAIR>(sb + static_cast<uint32_t>(i * p.b_box_bytes), &tmap_b, b_row + i * p.b_box_cols,
-                                    kb * kBlockK, fb);
-              }
+            };
+            copy(sa, sb, kb);
+            if constexpr (Cfg::kStageBlocks > 1) {
+              if (copies > 1) copy(sa + p.a_block_bytes, sb + Cfg::kBlockBytesB, kb + 1);
             }
             if (++stage == stages) {
               stage = 0;
@@ -1706,10 +1715,10 @@ bool encode_map(CUtensorMap* map, const MapKey& key_in) {
 // e4m3 matrix of `rows` rows (M or N) and K columns. K-major (K contiguous, row pitch ld): box = 128 bytes of
 // K x box_rows rows, 128-byte swizzle. MN-major (rows contiguous, ld bytes between consecutive k): box =
 // box_rows (128 or 64) bytes of rows x 128 k, swizzle span = the box's inner extent.
-// `blocks`: K blocks per copy. K-major: K is then two dimensions, the byte of a block and the block, so that a box holds
-// one K block's tile behind the other. MN-major: a box of that many times 128 k.
+// `blocks`: K blocks per copy. Where a stage has several (`by_block`), K is two dimensions of a K-major operand, the byte of a
+// block and the block, so that a box holds one K block's tile behind the other. MN-major: a box of that many times 128 k.
 bool encode_operand_map(CUtensorMap* map, const void* base, int rows, int K, long long ld, int box_rows,
-                        bool mn_major, int blocks) {
+                        bool mn_major, bool by_block, int blocks) {
   MapKey k;
   memset(&k, 0, sizeof(k));
   k.base = base;
@@ -1719,7 +1728,7 @@ bool encode_operand_map(CUtensorMap* map, const void* base, int rows, int K, lon
   k.strides[0] = static_cast<cuuint64_t>(ld);
   k.box[0] = static_cast<cuuint32_t>(mn_major ? box_rows : kBlockK);
   k.box[1] = static_cast<cuuint32_t>(mn_major ? blocks * kBlockK : box_rows);
-  if (!mn_major && blocks > 1) {
+  if (!mn_major && by_block) {
     k.rank = 3;
     k.dims[0] = kBlockK;
     k.dims[2] = static_cast<cuuint64_t>(K / kBlockK);
@@ -1752,7 +1761,7 @@ bool encode_output_map(CUtensorMap* map, void* base, int M, int N, long long ldc
 // Grouped operands: e4m3 [groups][rows][K] with K contiguous, row pitch ld and group pitch lg (bytes);
 // box = 128 bytes of K x box_rows rows x `blocks` K blocks of one group.
 bool encode_grouped_operand_map(CUtensorMap* map, const void* base, int groups, int rows, int K, long long ld,
-                                long long lg, int box_rows, int blocks) {
+                                long long lg, int box_rows, bool by_block, int blocks) {
   MapKey k;
   memset(&k, 0, sizeof(k));
   k.base = base;
@@ -1762,9 +1771,9 @@ bool encode_grouped_operand_map(CUtensorMap* map, const void* base, int groups, 
     if (d > 0) k.strides[d - 1] = static_cast<cuuint64_t>(stride);
     k.box[d++] = static_cast<cuuint32_t>(box);
   };
-  dimension(blocks > 1 ? kBlockK : K, 1, kBlockK);
+  dimension(by_block ? kBlockK : K, 1, kBlockK);
   dimension(rows, ld, box_rows);
-  if (blocks > 1) dimension(K / kBlockK, kBlockK, blocks);
+  if (by_block) dimension(K / kBlockK, kBlockK, blocks);
   dimension(groups, lg, 1);
   k.rank = d;
   k.dtype = CU_TENSOR_MAP_DATA_TYPE_UINT8;
@@ -1833,6 +1842,21 @@ constexpr int kMaxSmem = 232448;  // 227 KiB opt-in limit per CTA on sm_100
 int tmem_bufs_in_use(int block_n, int stages) {
   const int d = tmem_bufs_for(block_n);
   return d < stages ? d : stages;
+}
+
+// K blocks per copy: all of a stage's, which halves the producer's copies, but one at a time where a K range ends in half a
+// stage and is short: the other half of a box is loaded (or filled with zeros) for nothing then, and in a range of one to fifteen
+// blocks that is more than the further copies cost (two blocks a copy / one: 208 x 1008 x 384 MN-major 4.94 / 4.82 us, 224 x 2580 x
+// 384 4.79 / 4.65, 500 x 700 x 640 4.81 / 4.66, 128 x 3296 x 128 MN-major 3.91 / 3.78; seven blocks a range, 128 x 576 x 7168 in
+// clusters of eight, 7.73 / 7.66).
+int box_blocks_for(int block_n, int kblocks, int split) {
+  const int blocks = stage_blocks_for(block_n);
+  if (blocks == 1 || (kblocks + split - 1) / split > 15) return blocks;
+  for (int i = 0; i < split; ++i) {
+    const long long first = static_cast<long long>(i) * kblocks / split, end = static_cast<long long>(i + 1) * kblocks / split;
+    if ((end - first) % blocks != 0) return 1;
+  }
+  return blocks;
 }
 
 // A plan counts its ring in K blocks; where a stage has two, an odd last one is left unused.
@@ -2272,9 +2296,10 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   const OperandLayout la = operand_layout(a_mn, kBlockM);
   const OperandLayout lb = operand_layout(b_mn, b_box_rows_for(pl.block_n, pl.cta_pair));
   const int a_box = a_mn ? la.box_cols : a_box_rows_for(M);
-  const int blocks = stage_blocks_for(pl.block_n);
-  if (!encode_operand_map(&map_a, a, M, K, lda, a_box, a_mn, blocks)) return B200_FP8_MM_ERR_DRIVER;
-  if (!encode_operand_map(&map_b, b, N, K, ldb, lb.box_cols, b_mn, blocks)) return B200_FP8_MM_ERR_DRIVER;
+  const int blocks = box_blocks_for(pl.block_n, kblocks, pl.full_tiles < pl.tiles ? pl.split_k : 1);
+  const bool by_block = stage_blocks_for(pl.block_n) > 1;  // (the kernel's loads have as many coordinates as the maps have dimensions)
+  if (!encode_operand_map(&map_a, a, M, K, lda, a_box, a_mn, by_block, blocks)) return B200_FP8_MM_ERR_DRIVER;
+  if (!encode_operand_map(&map_b, b, N, K, ldb, lb.box_cols, b_mn, by_block, blocks)) return B200_FP8_MM_ERR_DRIVER;
 
   KernelParams kp;
   memset(&kp, 0, sizeof(kp));
@@ -2301,7 +2326,8 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
   kp.stages = ring_stages(pl);
   // (an MN-major a comes in boxes of 128 rows, whatever M is)
   const int a_rows = a_mn ? kBlockM : a_box;
-  kp.stage_tx = static_cast<uint32_t>(blocks * (a_rows + b_box_rows_for(pl.block_n, pl.cta_pair)) * kBlockK);
+  kp.box_blocks = blocks;
+  kp.copy_tx = static_cast<uint32_t>(blocks * (a_rows + b_box_rows_for(pl.block_n, pl.cta_pair)) * kBlockK);
   kp.a_block_bytes = static_cast<uint32_t>(a_rows * kBlockK);
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, kp.stages);
   kp.store_bufs = store_bufs;
@@ -2393,7 +2419,7 @@ int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUte
 // Cost of a grouped launch with row counts, which are device memory and unknown here: rated over loads from 1/8 to all of M,
 // and, at half the weight, with every group full. What a tile of a grouped kernel costs beside its K blocks is more than
 // in the plain kernels, most of all for pairs. (graph, us, tile shape chosen for full groups / this way: 8 x 1024 x 2048 x 7168
-// with loads of 1/8 .. 8/8 98 / 76, 16 x 300 x 1024 x 2048 24.9 / 18.8, 10 x 500 x 3520 x 384 21.2 / 17.1; every group full
+// with loads of 1/8 .. 8/8 102 / 75, 16 x 300 x 1024 x 2048 25.8 / 20.8, 10 x 500 x 3520 x 384 24.3 / 17.2; every group full
 // 128 / 138, half full 70 / 75.)
 double uneven_cost(int groups, int M, int N, int kblocks, int sm_count, int bn, int pair) {
   const int tile_m = pair ? 2 * kBlockM : kBlockM, units = pair ? sm_count / 2 : sm_count;
@@ -2479,10 +2505,11 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
     memset(&map_c, 0, sizeof(map_c));
   }
   const int a_box = a_box_rows_for(M);
-  const int blocks = stage_blocks_for(pl.block_n);
-  if (!encode_grouped_operand_map(&map_a, a, groups, M, K, lda, a_g, a_box, blocks)) return B200_FP8_MM_ERR_DRIVER;
+  const int blocks = box_blocks_for(pl.block_n, K / kBlockK, 1);
+  const bool by_block = stage_blocks_for(pl.block_n) > 1;
+  if (!encode_grouped_operand_map(&map_a, a, groups, M, K, lda, a_g, a_box, by_block, blocks)) return B200_FP8_MM_ERR_DRIVER;
   const int b_rows_per_cta = b_box_rows_for(pl.block_n, pl.cta_pair);
-  if (!encode_grouped_operand_map(&map_b, b, groups, N, K, ldb, b_g, b_rows_per_cta, blocks)) return B200_FP8_MM_ERR_DRIVER;
+  if (!encode_grouped_operand_map(&map_b, b, groups, N, K, ldb, b_g, b_rows_per_cta, by_block, blocks)) return B200_FP8_MM_ERR_DRIVER;
 
   const OperandLayout la = operand_layout(false, kBlockM);
   const OperandLayout lb = operand_layout(false, b_rows_per_cta);
@@ -2506,7 +2533,8 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   kp.full_tiles = groups * kp.tiles_m * kp.tiles_n;
   kp.kblocks = K / kBlockK;
   kp.stages = ring_stages(pl);
-  kp.stage_tx = static_cast<uint32_t>(blocks * (a_box + b_rows_per_cta) * kBlockK);
+  kp.box_blocks = blocks;
+  kp.copy_tx = static_cast<uint32_t>(blocks * (a_box + b_rows_per_cta) * kBlockK);
   kp.a_block_bytes = static_cast<uint32_t>(a_box * kBlockK);
   kp.tmem_bufs = tmem_bufs_in_use(pl.block_n, kp.stages);
   kp.store_bufs = store_bufs;
