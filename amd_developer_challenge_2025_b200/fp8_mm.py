@@ -363,8 +363,8 @@ def host_ranges(m: int, n: int, k: int, chunk_rows: int = 1024) -> tuple[bool, l
         parts = max(2 + moved // HOST_FURTHER_RANGE_BYTES, -(-extent // chunk_rows))
         rows = -(-extent // (parts * SCALE_BLOCK)) * SCALE_BLOCK
         inner = list(range(rows, extent, rows))
-    if by_columns:
-        inner = [r // SCALE_BLOCK * SCALE_BLOCK for r in inner]
+    if by_columns:  # onto whole scale blocks; the last cut may fall together with the one before it
+        inner = sorted({r // SCALE_BLOCK * SCALE_BLOCK for r in inner})
     return by_columns, [0] + inner + [extent]
 
 

@@ -6,21 +6,35 @@ import amd_developer_challenge_2025_b200 as pkg
 from amd_developer_challenge_2025_b200.fp8_mm import HOST_RANGE_BYTES, check_device_status, host_ranges
 
 
+def covers(m, n, k, chunk):
+    by_columns, cuts = host_ranges(m, n, k, chunk)
+    extent = n if by_columns else m
+    assert cuts[0] == 0 and cuts[-1] == extent and all(x < y for x, y in zip(cuts, cuts[1:])), (m, n, k, chunk, cuts)
+    if by_columns:  # the smaller operand goes first; blocks of columns start on whole scale blocks
+        assert n > m and all(x % 128 == 0 for x in cuts[:-1]), (m, n, k, chunk, cuts)
+    if m * k + n * k + 2 * m * n < HOST_RANGE_BYTES:
+        assert len(cuts) == 2
+
+
 def test_cuts_cover_the_streamed_operand():
     for m, n, k in ((1, 1, 128), (2048, 4608, 7168), (4608, 2048, 7168), (300, 4096, 1024), (1112, 4288, 2816), (700, 4305, 2816), (8192, 4608, 7168)):
         for chunk in (100, 256, 1024, 4096):
-            by_columns, cuts = host_ranges(m, n, k, chunk)
-            extent = n if by_columns else m
-            assert cuts[0] == 0 and cuts[-1] == extent and all(x < y for x, y in zip(cuts, cuts[1:]))
-            if by_columns:  # the smaller operand goes first; blocks of columns start on whole scale blocks
-                assert n > m and all(x % 128 == 0 for x in cuts[:-1])
-            if m * k + n * k + 2 * m * n < HOST_RANGE_BYTES:
-                assert len(cuts) == 2
+            covers(m, n, k, chunk)
+
+
+@pytest.mark.parametrize("m,k", [(1, 7168), (512, 1024), (2048, 7168), (4096, 2048)])
+@pytest.mark.parametrize("chunk", [128, 256, 384, 1000, 1024, 2048])
+def test_cuts_at_every_extent(m, k, chunk):
+    """Both operands streamed, at every extent: rounding may not bring two cuts of columns together (2048 x 4650 x 7168)."""
+    for extent in range(1, 12001):
+        covers(m, extent, k, chunk)
+        covers(extent, m, k, chunk)
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k,phase,chunk", [(5, 96, 256, 0, 1024), (40, 2048, 1024, 0, 256), (200, 2112, 1024, 64, 256), (130, 2100, 1024, 96, 256),
-                                               (1500, 576, 1024, 32, 256), (640, 1999, 640, 0, 100), (600, 4096, 1152, 0, 1024), (700, 4288, 1152, 64, 1024)])
+                                               (1500, 576, 1024, 32, 256), (640, 1999, 640, 0, 100), (600, 4096, 1152, 0, 1024), (700, 4288, 1152, 64, 1024), (2048, 4650, 7168, 0, 1024),
+                                               (2048, 4640, 7168, 32, 1024)])
 def test_ranges_equal_the_whole_problem(m, n, k, phase, chunk):
     a, b, a_s, _, _ = pkg.make_inputs(m, n, k, seed=m + n)
     g = torch.Generator().manual_seed(n)
