@@ -5,6 +5,7 @@ Mirrors the reference's pybind launcher `fp8_mm(a, b, as, bs, c, c_tmp)`
 from __future__ import annotations
 
 import ctypes
+import operator
 import threading
 from dataclasses import dataclass
 
@@ -351,7 +352,8 @@ def host_ranges(m: int, n: int, k: int, chunk_rows: int = 1024) -> tuple[bool, l
 
     Nothing can travel back before one operand is there in full: that is the smaller one (1112 x 4305 x 2816 by columns 455 us, by
     rows 497; 300 x 4608 x 1024 203 and 216), and the larger one arrives in equal ranges of at most `chunk_rows` rows (of b: columns
-    of c), or with short ranges at both ends where there are many large ones."""
+    of c), rounded up to whole scale blocks, or, where there are many large ones, in ranges of `chunk_rows` with a short one of about
+    256 at each end. Small problems come in one range, whatever `chunk_rows` is."""
     by_columns = n > m and chunk_rows > 0 and chunk_rows % SCALE_BLOCK == 0
     extent = n if by_columns else m
     moved = m * k + n * k + 2 * m * n
@@ -368,13 +370,24 @@ def host_ranges(m: int, n: int, k: int, chunk_rows: int = 1024) -> tuple[bool, l
     return by_columns, [0] + inner + [extent]
 
 
+def _range_rows(m: int, chunk_rows) -> int:
+    """`chunk_rows` as a positive whole number. Problems of up to 512 rows are never cut by rows and take any value: what is no
+    positive whole number bounds nothing there."""
+    try:
+        rows = operator.index(chunk_rows)
+    except TypeError:
+        rows = 0
+    _check(rows >= 1 or m <= 512, "chunk_rows must be a whole number of at least 1")
+    return rows if rows >= 1 else 1 << 30
+
+
 def fp8_mm_host(a, b, a_scale, b_scale, c, device="cuda", n_phase: int = 0, chunk_rows: int = 1024):
     """The same operator for HOST tensors (pinned memory for full speed): returns c, filled, when done.
 
     The smaller operand and the scales are copied to `device` first; the larger one is then streamed in row ranges
     (`host_ranges`), each range's GEMM runs as soon as its rows have landed, and its part of c is copied back while later
     ranges are still arriving, so both directions of the host link and the SMs work at the same time (three
-    streams, events between them). Every range is an independent GEMM with the plan the
+    streams, events between them). `chunk_rows` bounds the rows of a range (see `host_ranges`). Every range is an independent GEMM with the plan the
     library picks for its size; the result meets the same tolerance as one GEMM over the whole problem
     (and equals it bit for bit unless a range's plan splits K, which only changes the order in which K
     ranges are added). Device buffers are kept per device between calls of the same shape. This is the
@@ -388,6 +401,7 @@ def fp8_mm_host(a, b, a_scale, b_scale, c, device="cuda", n_phase: int = 0, chun
            and c.is_contiguous(), "host tensors must be contiguous")
     m, k = a.shape
     n = b.shape[0]
+    chunk_rows = _range_rows(m, chunk_rows)
     pipe = _host_pipelines.get(dev.index)
     if pipe is None:
         pipe = _host_pipelines[dev.index] = _HostPipeline(dev)

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 import amd_developer_challenge_2025_b200 as pkg
-from amd_developer_challenge_2025_b200.fp8_mm import HOST_RANGE_BYTES, check_device_status, host_ranges
+from amd_developer_challenge_2025_b200.fp8_mm import HOST_RANGE_BYTES, _range_rows, check_device_status, host_ranges
 
 
 def covers(m, n, k, chunk):
@@ -14,6 +14,8 @@ def covers(m, n, k, chunk):
         assert n > m and all(x % 128 == 0 for x in cuts[:-1]), (m, n, k, chunk, cuts)
     if m * k + n * k + 2 * m * n < HOST_RANGE_BYTES:
         assert len(cuts) == 2
+    if len(cuts) > 2:
+        assert max(y - x for x, y in zip(cuts, cuts[1:])) <= max(-(-chunk // 128) * 128, 256), (m, n, k, chunk, cuts)
 
 
 def test_cuts_cover_the_streamed_operand():
@@ -29,6 +31,16 @@ def test_cuts_at_every_extent(m, k, chunk):
     for extent in range(1, 12001):
         covers(m, extent, k, chunk)
         covers(extent, m, k, chunk)
+
+
+@pytest.mark.parametrize("chunk", [0, -7, None, 512.0])
+def test_what_bounds_nothing(chunk):
+    """Up to 512 rows, which are never cut by rows, any value is taken (300 x 640 x 7168 divided by zero); beyond, it is refused."""
+    for m, n, k in ((300, 640, 7168), (512, 96, 7168), (512, 4608, 7168)):
+        covers(m, n, k, _range_rows(m, chunk))
+    with pytest.raises(ValueError):
+        _range_rows(513, chunk)
+    assert _range_rows(513, 1024) == 1024 and _range_rows(5, 1) == 1
 
 
 @pytest.mark.gpu
@@ -48,6 +60,20 @@ def test_ranges_equal_the_whole_problem(m, n, k, phase, chunk):
         check_device_status()
         # a range whose plan splits K adds its partial sums in another order: one rounding of bf16
         torch.testing.assert_close(out.float(), whole.cpu().float(), rtol=2 ** -7, atol=1e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scales", [torch.float32, torch.float64])  # the plain call and the converting one
+def test_chunk_rows_of_zero(scales):
+    for m, n in ((300, 640), (513, 640)):
+        a, b, a_s, b_s, c = pkg.make_inputs(m, n, 7168, seed=m)
+        want = pkg.fp8_mm_host(a, b, a_s, b_s, torch.zeros_like(c))
+        call = lambda: pkg.fp8_mm_host(a, b, a_s.to(scales), b_s, c, chunk_rows=0)
+        if m <= 512:
+            torch.testing.assert_close(call().float(), want.float(), rtol=2 ** -7, atol=1e-3)
+        else:
+            with pytest.raises(ValueError):
+                call()
 
 
 @pytest.mark.gpu
