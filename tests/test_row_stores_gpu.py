@@ -1,6 +1,6 @@
-"""Rows of c that the TMA store cannot address (odd pitch or base) and tiles that a group's row count cuts short leave
-through shared memory row by row. Each run is compared bit for bit with the same plan writing an aligned c, which the
-parity tests hold against the CPU oracle; the elements around c must keep their value."""
+"""Rows of c that the TMA store cannot write (odd pitch or base, a row length that is no multiple of 8) and tiles that a group's
+row count cuts short leave straight from registers. Each run is compared bit for bit with the same plan's TMA store: an aligned c of
+N up to the next multiple of 8, which the parity tests hold against the CPU oracle. The elements around c must keep their value."""
 import pytest
 import torch
 
@@ -29,8 +29,9 @@ def untouched(buf, m, n, pitch, offset):
 def test_unaligned_rows_equal_the_aligned_run(block_n, pair, m, n, pad, offset):
     plan = Plan(block_n=block_n, cta_pair=pair, split_k=1)
     a, b, a_s, b_s, _ = pkg.make_inputs(m, n, 384, seed=m + n, device="cuda")
-    wide = torch.zeros(m, (n + 15) // 8 * 8, dtype=torch.bfloat16, device="cuda")
-    fp8_mm(a, b, a_s, b_s, wide[:, :n], plan=plan)
+    more = torch.zeros(-n % 8, 384, dtype=torch.uint8, device="cuda")  # (no further scale block and no further tile)
+    wide = torch.zeros(m, (n + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")
+    fp8_mm(a, torch.cat((b.view(torch.uint8), more)).view(b.dtype), a_s, b_s, wide, plan=plan)
     pitch = n + pad
     buf, c = inside(m, n, pitch, offset)
     fp8_mm(a, b, a_s, b_s, c, plan=plan)

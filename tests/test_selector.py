@@ -24,8 +24,7 @@ def test_plans(built_library, m, n, k):
     assert p.grid <= 148 and p.smem_bytes <= 232448
     if p.full_tiles == p.tiles:
         assert p.split_k == 1 and p.grid == min(p.tiles, units) * (2 if p.cta_pair else 1)
-        if p.cta_pair and p.block_n == 64:
-            assert k // 128 >= 20
+        assert not (p.cta_pair and p.block_n == 64)  # (such a plan becomes single CTAs)
     elif p.full_tiles == 0 and not p.cta_pair and p.block_n <= 128 and p.split_k <= 8 and p.tiles <= CLUSTERS[p.split_k]:
         assert p.grid == p.tiles * p.split_k and p.split_k * 2 <= k // 128       # one cluster per tile, all at once
         assert p.stages * (128 + p.block_n) * 128 >= 128 * (p.block_n + 4) * 4   # the ring holds a partial tile
