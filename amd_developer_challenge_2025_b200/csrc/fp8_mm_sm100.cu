@@ -2008,10 +2008,11 @@ Candidate evaluate(int M, int N, int kblocks, int sm_count, int bn, int pair, in
   return best;
 }
 
-// 128-wide single CTAs with one tile each: nothing runs under the TMA store of a tile, so its rows leave straight from registers
-// (store_row), and without the second staging buffer the ring has six stages for four, which pays from about as many K blocks on
-// (2048 x 512 x 7168 24.1 -> 20.1 us, 369 x 3196 x 1792 10.1 -> 9.0, 1500 x 1000 x 2048 10.4 -> 9.9). With several tiles a CTA
-// the TMA store is ahead (2048 x 7168 x 512 19.1 against 20.9).
+// 128-wide single CTAs with one tile each: nothing runs under the TMA store of a tile, so one staging buffer does, and without the
+// second the ring has six stages for four, which pays from about as many K blocks on (one buffer and six stages / two and four:
+// forced on 2048 x 512 x 7168 20.0 / 21.8 us, 369 x 3200 x 1792 8.5 / 8.7, 1500 x 1000 x 2048 10.0 / 10.1, 1024 x 2048 x 1024 7.2 / 7.3,
+// grouped 4 x 128 x 2048 x 7168 21.2 / 26.8, 8 x 256 x 1024 x 2048 10.3 / 11.3). Rows straight from registers are slower: 8.9, 7.9
+// and, at 1152 x 1536 x 4096, 16.4 against 16.2. With several tiles a CTA two buffers are ahead (2048 x 7168 x 512 19.1 against 20.9).
 bool long_ring(int bn, int pair, int split, int tiles, int units, int kblocks) {
   return bn == 128 && !pair && split == 1 && tiles <= units && kblocks > 6;
 }
@@ -2287,7 +2288,6 @@ int run(const void* a, const void* b, const float* a_scale, const float* b_scale
 
   CUtensorMap map_a, map_b, map_c;
   int store_bufs = tma_store_fits(c, N, ldc, 0) ? pl.store_bufs : 0;
-  if (forced_in == nullptr && long_ring(pl.block_n, pl.cta_pair, pl.split_k, pl.tiles, sm_count, kblocks)) store_bufs = 0;
   if (store_bufs > 0) {
     if (!encode_output_map(&map_c, c, M, N, ldc)) return B200_FP8_MM_ERR_DRIVER;
   } else {
