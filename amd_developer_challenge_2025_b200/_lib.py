@@ -26,6 +26,7 @@ EXPORTS = (
     "b200_fp8_mm_static_scratch_limit",
     "b200_fp8_mm_selftest_wait_expiry",
     "b200_fp8_mm_host_ranges",
+    "b200_fp8_mm_grouped_describe",
     "b200_fp8_mm_workspace_bytes",
     "b200_fp8_mm_plan_workspace_bytes",
     "b200_fp8_mm_describe",
@@ -134,6 +135,8 @@ def load() -> ctypes.CDLL:
     lib.b200_fp8_mm_host_ranges.argtypes = ([ctypes.c_void_p] * 5 + [ctypes.c_int] * 5 + [ctypes.POINTER(ctypes.c_int), ctypes.c_int]
                                             + [ctypes.c_void_p] * 6 + [ctypes.c_size_t] + [ctypes.c_void_p] * 5)
     lib.b200_fp8_mm_host_ranges.restype = ctypes.c_int
+    lib.b200_fp8_mm_grouped_describe.argtypes = [ctypes.c_int] * 6 + [ctypes.POINTER(CPlan)]
+    lib.b200_fp8_mm_grouped_describe.restype = ctypes.c_int
     lib.b200_fp8_mm_static_scratch_limit.argtypes = []
     lib.b200_fp8_mm_static_scratch_limit.restype = ctypes.c_size_t
     lib.b200_fp8_mm_workspace_bytes.argtypes = [ctypes.c_int] * 3

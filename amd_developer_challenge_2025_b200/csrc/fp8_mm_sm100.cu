@@ -2416,26 +2416,81 @@ int launch(KernelFn fn, const b200_fp8_mm_plan& pl, int cluster_ctas, const CUte
   return B200_FP8_MM_OK;
 }
 
-// Cost of a grouped launch with row counts, which are device memory and unknown here: rated over loads from 1/8 to all of M,
-// and, at half the weight, with every group full. What a tile of a grouped kernel costs beside its K blocks is more than
-// in the plain kernels, most of all for pairs. (graph, us, tile shape chosen for full groups / this way: 8 x 1024 x 2048 x 7168
-// with loads of 1/8 .. 8/8 102 / 75, 16 x 300 x 1024 x 2048 25.8 / 20.8, 10 x 500 x 3520 x 384 24.3 / 17.2; every group full
-// 128 / 138, half full 70 / 75.)
-double uneven_cost(int groups, int M, int N, int kblocks, int sm_count, int bn, int pair) {
-  const int tile_m = pair ? 2 * kBlockM : kBlockM, units = pair ? sm_count / 2 : sm_count;
-  const WidthCost wc = width_cost(bn, pair);
-  const double extra = pair ? 2000.0 : (bn == 256 ? 500.0 : (bn == 192 ? 1500.0 : 0.0));
-  long long eighths = 0;  // tile rows of eight groups, one of each load
-  for (int i = 1; i <= 8; ++i) eighths += ceil_div(ceil_div(M, 8) * i < M ? ceil_div(M, 8) * i : M, tile_m);
-  auto waves = [&](double tile_rows) { return ceil(tile_rows * ceil_div(N, bn) / units - 1e-9); };
-  const double uneven = waves(ceil(static_cast<double>(groups) * static_cast<double>(eighths) / 8.0));
-  const double full = waves(static_cast<double>(groups) * ceil_div(M, tile_m));
-  return (uneven + 0.5 * full) * (kblocks * wc.per_kblock + wc.per_tile + extra);
+// The single-CTA width that a grouped launch with row counts uses in place of pairs, or 0.
+//
+// Loads that leave the pairs' 256-row tiles half empty cost them up to 40 %; even loads cost single CTAs what pairs save per K block.
+// The counts are device memory, so the shape has to do for any of them: single CTAs take the pairs' place where the model finds
+// them less than 3 % dearer with every group full and with every group half full, and cheaper with loads spread over 1/8 .. 8/8.
+// (us, pairs / single 256-wide CTAs, every group full, half full, spread: 10 x 500 x 3520 x 384 19.6 / 19.3, 17.9 / 14.8, 22.2 / 17.6;
+// 16 x 1024 x 2048 x 1024 45.7 / 47.6, 29.0 / 30.0, 40.8 / 31.1; 12 x 768 x 2304 x 512 25.1 / 25.5, 27.6 / 17.5, 24.4 / 19.2. The pairs
+// stay at 8 x 1024 x 2048 x 7168: 128 / 135, 67 / 72, 97 / 76. Rated mostly by spread loads, that one gave up 6 % of even loads and
+// 8 x 512 x 2048 x 7168, as 192-wide pairs, a fifth to a third: 68 -> 84 full, 38 -> 58 half full.)
+int single_for_pairs(int groups, int M, int N, int kblocks, int sm_count, int pair_n) {
+  enum Load { kFull, kHalf, kSpread };
+  auto time = [&](int bn, int pair, Load load) {
+    const int tile_m = pair ? 2 * kBlockM : kBlockM, units = pair ? sm_count / 2 : sm_count;
+    long long rows = 0;  // tile rows of eight groups
+    for (int i = 1; i <= 8; ++i) {
+      const int loaded = load == kFull ? M : (load == kHalf ? ceil_div(M, 2) : ceil_div(M, 8) * i);
+      rows += ceil_div(loaded < M ? loaded : M, tile_m);
+    }
+    const double tiles = ceil(static_cast<double>(groups) * static_cast<double>(rows) / 8.0) * ceil_div(N, bn);
+    // What a tile takes in a grouped kernel beside its K blocks is more than in the plain ones, most of all for pairs: about as much
+    // in 20 problems of 2 to 64 groups with six kinds of counts. A launch takes some 5000 clocks whatever it does.
+    const WidthCost wc = width_cost(bn, pair);
+    const double extra = pair ? 2000.0 : (bn == 256 ? 500.0 : (bn == 192 ? 1500.0 : 1000.0));
+    return 5000.0 + ceil(tiles / units - 1e-9) * (kblocks * wc.per_kblock + wc.per_tile + extra);
+  };
+  const double full = time(pair_n, 1, kFull), half = time(pair_n, 1, kHalf);
+  double best = time(pair_n, 1, kSpread) / 1.02;
+  int instead = 0;
+  for (int bn = 256; bn >= 128; bn -= 64) {
+    const double spread = time(bn, 0, kSpread);
+    if (spread >= best || time(bn, 0, kFull) > 1.03 * full || time(bn, 0, kHalf) > 1.03 * half) continue;
+    best = spread;
+    instead = bn;
+  }
+  return instead;
 }
 
-// Grouped launch: `groups` problems of the same N and K in one kernel. Every tile is a whole tile (no split-K); its shape
-// is chosen as for one GEMM with all groups' row blocks stacked, CTA pairs only where a group's rows fill their tiles; with row
-// counts by uneven_cost().
+// The plan of a grouped launch: `groups` problems of the same N and K in one kernel. Every tile is a whole tile (no split-K); its
+// shape is chosen as for one GEMM with all groups' row blocks stacked, CTA pairs only where a group's rows fill their tiles; with
+// row counts see single_for_pairs().
+int plan_grouped(int groups, int M, int N, int K, int sm_count, bool with_counts, const b200_fp8_mm_plan* forced_in,
+                 b200_fp8_mm_plan* out) {
+  b200_fp8_mm_plan forced;
+  if (forced_in != nullptr) {
+    if (forced_in->split_k > 1) return B200_FP8_MM_ERR_PLAN;
+    forced = *forced_in;
+  } else {
+    memset(&forced, 0, sizeof(forced));
+  }
+  forced.split_k = 1;
+  // CTA pairs work on 256-row tiles inside each group: considered when a group's rows fill them to at
+  // least 7/8 (or when forced), and only at the widths that have a paired grouped kernel.
+  const int rows256 = ceil_div(M, 2 * kBlockM) * 2 * kBlockM;
+  const bool pair_fits = (rows256 - M) * 8 <= M;
+  if (forced.cta_pair == 0 && !pair_fits) forced.cta_pair = -1;
+  choose_plan(groups * rows256, N, K, sm_count, &forced, out);
+  if (out->cta_pair && out->block_n != 192 && out->block_n != 256) {
+    if (forced_in != nullptr && forced_in->cta_pair > 0) return B200_FP8_MM_ERR_PLAN;
+    forced.cta_pair = -1;
+  }
+  if (!out->cta_pair || forced.cta_pair < 0) {
+    forced.cta_pair = -1;
+    choose_plan(groups * ceil_div(M, kBlockM) * kBlockM, N, K, sm_count, &forced, out);
+  }
+  if (with_counts && forced_in == nullptr && out->cta_pair) {
+    const int instead = single_for_pairs(groups, M, N, K / kBlockK, sm_count, out->block_n);
+    if (instead != 0) {
+      forced.block_n = instead;
+      forced.cta_pair = -1;
+      choose_plan(groups * ceil_div(M, kBlockM) * kBlockM, N, K, sm_count, &forced, out);
+    }
+  }
+  return B200_FP8_MM_OK;
+}
+
 int run_grouped(const void* a, const void* b, const float* a_scale, const float* b_scale, void* c, int groups, int M,
                 int N, int K, long long lda, long long a_g, long long ldb, long long b_g, long long sa_g,
                 long long sa_m, long long sa_k, long long sb_g, long long sb_n, long long sb_k, long long ldc,
@@ -2453,45 +2508,9 @@ int run_grouped(const void* a, const void* b, const float* a_scale, const float*
   const int sm_count = device_sm_count();
   if (sm_count <= 0) return B200_FP8_MM_ERR_DRIVER;
 
-  b200_fp8_mm_plan forced;
-  if (forced_in != nullptr) {
-    if (forced_in->split_k > 1) return B200_FP8_MM_ERR_PLAN;
-    forced = *forced_in;
-  } else {
-    memset(&forced, 0, sizeof(forced));
-  }
-  forced.split_k = 1;
-  // CTA pairs work on 256-row tiles inside each group: considered when a group's rows fill them to at
-  // least 7/8 (or when forced), and only at the widths that have a paired grouped kernel.
-  const int rows256 = ceil_div(M, 2 * kBlockM) * 2 * kBlockM;
-  const bool pair_fits = (rows256 - M) * 8 <= M;
-  if (forced.cta_pair == 0 && !pair_fits) forced.cta_pair = -1;
   b200_fp8_mm_plan pl;
-  choose_plan(groups * rows256, N, K, sm_count, &forced, &pl);
-  if (pl.cta_pair && pl.block_n != 192 && pl.block_n != 256) {
-    if (forced_in != nullptr && forced_in->cta_pair > 0) return B200_FP8_MM_ERR_PLAN;
-    forced.cta_pair = -1;
-  }
-  if (!pl.cta_pair || forced.cta_pair < 0) {
-    forced.cta_pair = -1;
-    choose_plan(groups * ceil_div(M, kBlockM) * kBlockM, N, K, sm_count, &forced, &pl);
-  }
-  if (m_valid != nullptr && forced_in == nullptr) {
-    double best = 1e300;
-    b200_fp8_mm_plan shape;
-    memset(&shape, 0, sizeof(shape));
-    shape.split_k = 1;
-    for (int pair = pair_fits ? 1 : 0; pair >= 0; --pair) {
-      for (int bn = 256; bn >= (pair ? 192 : 64); bn -= 64) {
-        const double cost = uneven_cost(groups, M, N, K / kBlockK, sm_count, bn, pair);
-        if (cost >= best) continue;
-        best = cost;
-        shape.block_n = bn;
-        shape.cta_pair = pair ? 1 : -1;
-      }
-    }
-    choose_plan(groups * (shape.cta_pair > 0 ? rows256 : ceil_div(M, kBlockM) * kBlockM), N, K, sm_count, &shape, &pl);
-  }
+  const int planned = plan_grouped(groups, M, N, K, sm_count, m_valid != nullptr, forced_in, &pl);
+  if (planned != B200_FP8_MM_OK) return planned;
   if (!plan_is_supported(pl, K / kBlockK) || pl.split_k != 1) return B200_FP8_MM_ERR_PLAN;
   const int tiles_m = ceil_div(M, pl.cta_pair ? 2 * kBlockM : kBlockM);
   KernelFn fn = kernel_for(pl.block_n, pl.cta_pair, kGrouped);
@@ -2709,6 +2728,13 @@ int b200_fp8_mm_grouped(const void* a, const void* b, const float* a_scale, cons
                         void* stream, const b200_fp8_mm_plan* forced) {
   return run_grouped(a, b, a_scale, b_scale, c, groups, M, N, K, lda, a_g, ldb, b_g, sa_g, sa_m, sa_k, sb_g, sb_n,
                      sb_k, ldc, c_g, m_valid, device_status, stream, forced);
+}
+
+int b200_fp8_mm_grouped_describe(int groups, int M, int N, int K, int with_counts, int sm_count, b200_fp8_mm_plan* out) {
+  if (out == nullptr) return B200_FP8_MM_ERR_NULL;
+  if (groups <= 0 || M <= 0 || N <= 0 || K <= 0 || (K % kBlockK) != 0 || static_cast<long long>(groups) * ceil_div(M, kBlockM) > (1 << 20))
+    return B200_FP8_MM_ERR_SHAPE;
+  return plan_grouped(groups, M, N, K, sm_count > 0 ? sm_count : 148, with_counts != 0, nullptr, out);
 }
 
 int b200_fp8_mm_host_ranges(const void* a, const void* b, const float* a_scale, const float* b_scale, void* c, int M, int N,

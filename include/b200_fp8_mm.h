@@ -243,6 +243,10 @@ int b200_fp8_mm_selftest_wait_expiry(const void* a, const void* b, const float* 
                                      unsigned long long wait_limit_ns, int skip_kblock,
                                      int* device_status, void* stream);
 
+/* The plan of a grouped launch, with or without row counts (block_n, cta_pair, stages, store_bufs; the other fields are those of one
+ * GEMM with all groups' row blocks stacked). sm_count 0: 148. Host arithmetic only. */
+int b200_fp8_mm_grouped_describe(int groups, int M, int N, int K, int with_counts, int sm_count, b200_fp8_mm_plan* out);
+
 /*
  * The GEMM for operands and result in host memory (pinned for full speed), contiguous: a [M,K], b [N,K], scales [M,K/128]
  * and [ceil((N+n_phase)/128),K/128], c [M,N]. One operand is copied to the device first; the other follows in `ranges` ranges of
