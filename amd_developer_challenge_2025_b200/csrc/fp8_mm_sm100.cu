@@ -17,8 +17,8 @@
 //               which both frees the stage for the producer and publishes the buffer to the
 //               promotion warps. It waits on ONE barrier per K block: a stage's "full" barrier also
 //               collects the promotion warps' release of the TMEM buffer that K block will
-//               overwrite (K block j uses stage j mod stages and buffer j mod buffers; a warp that
-//               has drained the buffer of K block j arrives on the barrier of K block j + buffers)
+//               overwrite (use j of the ring, one K block, or two at 64-wide tiles, takes stage j mod stages
+//               and buffer j mod buffers; a warp that has drained use j's buffer arrives on the barrier of use j + buffers)
 //   warp 2      allocates / frees TMEM; its first lane is a second MMA issuer at the narrow tiles (the
 //               two issuers take one K block each of a stage of two, or share the ring by stage, see issuer_walk.h)
 //   warp 3      scale loader: cp.async of the a_scale / b_scale values of FOUR K blocks at a time
@@ -82,7 +82,8 @@ __host__ __device__ constexpr int issuers_for(int block_n) { return block_n <= 1
 // through its barriers and copies (the producer needs about 420 clocks for its wait, expect_tx and two copies; the tensor core
 // 136, the operands' way into shared memory 390), so two of them share a stage: one wait, one expect_tx and two copies of the
 // producer, one wait and one release of the promotion warps for both. 2048 x 576 x 7168 18.1 -> 15.3 us, 32 x 576 x 1024 4.8 ->
-// 4.5. At 128 columns it was slower (8192 x 4608 x 7168 298 -> 304 us with single CTAs, 281 -> 280 with pairs; split in
+// 4.5, 128 x 2048 x 7168 16.7 -> 13.6; ranges of one, three and five blocks, whose last stage is half empty, are slower by 0.05 to 0.1 us
+// of 3.5 to 4.5. At 128 columns it was slower (8192 x 4608 x 7168 298 -> 304 us with single CTAs, 281 -> 280 with pairs; split in
 // clusters 256 x 1536 x 7168 11.2 -> 12.8): half as many stages fit, and the operands' way is what bounds it.
 __host__ __device__ constexpr int stage_blocks_for(int block_n) { return block_n == 64 ? 2 : 1; }
 // TMEM partial buffers, each for the K blocks of one stage (at most 512 columns in all).
@@ -1836,9 +1837,9 @@ int smem_bytes_for(int block_n, int stages, int pair, int store_bufs) {
 
 constexpr int kMaxSmem = 232448;  // 227 KiB opt-in limit per CTA on sm_100
 
-// K block j uses ring stage j mod stages and TMEM buffer j mod buffers; the two counts are independent
-// (the promotion warps release a buffer to the barrier of the stage that the K block `buffers` later will
-// use), except that a buffer cannot be re-used before its stage is: buffers <= stages.
+// Use j of the ring (one K block, or two at 64-wide tiles) takes stage j mod stages and TMEM buffer j mod buffers; the two counts
+// are independent (the promotion warps release a buffer to the barrier of the stage that the use `buffers` later will
+// take), except that a buffer cannot be re-used before its stage is: buffers <= stages.
 int tmem_bufs_in_use(int block_n, int stages) {
   const int d = tmem_bufs_for(block_n);
   return d < stages ? d : stages;
@@ -1847,8 +1848,9 @@ int tmem_bufs_in_use(int block_n, int stages) {
 // K blocks per copy: all of a stage's, which halves the producer's copies, but one at a time where a K range ends in half a
 // stage and is short: the other half of a box is loaded (or filled with zeros) for nothing then, and in a range of one to fifteen
 // blocks that is more than the further copies cost (two blocks a copy / one: 208 x 1008 x 384 MN-major 4.94 / 4.82 us, 224 x 2580 x
-// 384 4.79 / 4.65, 500 x 700 x 640 4.81 / 4.66, 128 x 3296 x 128 MN-major 3.91 / 3.78; seven blocks a range, 128 x 576 x 7168 in
-// clusters of eight, 7.73 / 7.66).
+// 384 4.79 / 4.65, 500 x 700 x 640 4.81 / 4.66, 128 x 3296 x 128 MN-major 3.91 / 3.78; even ranges gain 1 % at
+// most from single blocks and lose up to 17 %: 96 x 4096 x 1792 6.05 / 5.98, 8 x 1024 x 256 3.71 / 3.75, MN-major 32 x 576 x 1024 5.03 /
+// 5.19, 128 x 576 x 1536 5.46 / 6.39).
 int box_blocks_for(int block_n, int kblocks, int split) {
   const int blocks = stage_blocks_for(block_n);
   if (blocks == 1 || (kblocks + split - 1) / split > 15) return blocks;
@@ -1906,7 +1908,8 @@ size_t plan_workspace_bytes(const b200_fp8_mm_plan& pl) {
 // plan over the 36 benchmark shapes on B200. Per tile width 64/128/192/256: clocks per K block (bounded
 // by the promotion warps' chain of barrier probe, TMEM fetch and fmas, not by the tensor pipe), clocks
 // per tile for the bf16 output, and for split-K a constant plus a per-range cost of the fp32 round
-// trip and the last-arriver reduction.
+// trip and the last-arriver reduction. (64-wide tiles are rated as fitted with one K block a stage, here and in cluster_cost; with
+// two a stage a K block takes a quarter less, 345 clocks for 459 at 128 x 2048.)
 struct WidthCost {
   double per_kblock, per_tile, split_const, per_split;
 };
@@ -1914,9 +1917,9 @@ struct WidthCost {
 WidthCost width_cost(int bn, int pair) {
   // CTA pairs: each CTA loads half of the B tile, which pays per K block at the wide tiles (192: 5 % fewer
   // clocks than single CTAs, 256: 12 % fewer; K <= 512 loses 2-5 % to the dearer tile turnaround). At 128
-  // columns pairs measured slower throughout; at 64 columns they are 3-6 % faster when no tile is split (2048 x
-  // 576, 2048 x 512 and 512 x 1536 with K = 7168: one wave of 72, 64 and 48 pair tiles) and about 10 % slower
-  // with split K. Plans with a split-K tail measured about 7 % above this model, hence the larger constant.
+  // columns pairs measured slower throughout; at 64 columns about 10 % slower with split K, and unsplit they are rated 4 % below
+  // single CTAs, as they were with one K block a stage, and run as single CTAs (see choose_plan).
+  // Plans with a split-K tail measured about 7 % above this model, hence the larger constant.
   if (pair && bn == 192) return {775.0, 3600.0, 12000.0, 1000.0};
   if (pair && bn == 256) return {930.0, 3600.0, 14000.0, 1500.0};
   switch (bn) {
@@ -2066,8 +2069,8 @@ double choose_plan(int M, int N, int K, int sm_count, const b200_fp8_mm_plan* fo
   }
   if (best.bn == 0) best = Candidate{f_bn, f_pair > 0 ? 1 : 0, 1, 0, 0.0};  // invalid forced width
   // 64-wide pairs halve what a CTA loads of b per K block but take longer to start, to finish and to hand a K block over: single
-  // CTAs are faster (two K blocks a stage: 2048 x 576 x 7168 15.8 against 16.5 us, 512 x 1536 x 7168 15.0 against 15.9,
-  // 1024 x 1024 x 1024 5.6 against 6.4, 129 x 4099 x 2304 8.7 against 9.3).
+  // CTAs are faster (two K blocks a stage: 2048 x 576 x 7168 15.8 against 16.5 us, 512 x 1536 x 7168, forced, where 128-wide clusters
+  // run, 15.0 against 15.9, 1024 x 1024 x 1024 5.6 against 6.4, 129 x 4099 x 2304 8.7 against 9.3).
   // (They stay ahead of the wider tiles that the pair was ahead of: 909 x 2325 x 1152 10.0 us, 192-wide pairs 11.2. From here on
   // the cost is the single-CTA plan's own, so that it is what clusters have to beat.)
   if (f_pair < 0 && best.pair && best.bn == 64 && best.split == 1)

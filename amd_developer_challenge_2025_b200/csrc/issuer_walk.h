@@ -9,7 +9,9 @@
 #define ISSUER_WALK_FN inline
 #endif
 
-// K block j of a CTA's whole sequence lies in ring stage j mod stages and TMEM buffer j mod buffers. Issuer `me` of `issuers`
+// "Block" here is one use of the ring: a K block, or the two that share a stage at 64-wide tiles, where both MMA threads walk every
+// use (issuers = 1) and take a K block of it each.
+// Block j of a CTA's whole sequence lies in ring stage j mod stages and TMEM buffer j mod buffers. Issuer `me` of `issuers`
 // takes the blocks of stages me, me + issuers, ...: every issuers-th block while the number of stages is a multiple of
 // `issuers`, and at the end of an odd ring of two the next block follows at once.
 //
