@@ -1471,7 +1471,8 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
       // The TMA store clips at the tensor's edges only: a tile that a group's row count cuts short goes out
       // through the guarded plain stores instead.
       const bool tma_rows_ok = MODE != kGrouped || (it.m_limit == p.M) || (it.m0 + Cfg::kTileM <= it.m_limit);
-      if (__builtin_expect(do_store && p.store_bufs > 0 && tma_rows_ok, 1)) {
+      const bool by_tma = p.store_bufs > 0 && tma_rows_ok;
+      if (do_store && by_tma) {
         // bf16 tile -> swizzled staging -> TMA store, 32 columns at a time per warpgroup. The
         // 16-byte piece q of row r sits at r*64 + ((q ^ ((r >> 1) & 3)) * 16) (SWIZZLE_64B), which
         // spreads a warp's stores over all banks.
@@ -1538,7 +1539,10 @@ fp8_mm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gr
             if (wg_tid == 0 && *abort_flag == 0) store_box(ch, bufi);
           }
         }
-      } else if (do_store && ok) {
+      }
+      // (Not an `else`: one puts the code so that TMA-stored tiles are slower too, which no instruction of theirs explains: 526 x 2656 x 256
+      // 5.27 against 5.14 us, 1284 x 1512 x 512 6.32 / 6.24, 5030 x 832 x 256 7.02 / 6.91, MN-major 6144 x 3072 x 1536 35.9 / 35.4.)
+      if (do_store && ok && !by_tma) {
         const int at = it.m0 + static_cast<int>(cta_rank) * kBlockM + quarter * 32 + lane;
         if (at < it.m_limit)
           store_row<Cfg::kColsPerThread>(p.c + static_cast<long long>(it.group) * p.c_g + static_cast<long long>(at) * p.ldc + col0,
